@@ -193,19 +193,27 @@ struct dalm_handle {
         stream = nullptr;
     }
 
+    // Device memory of the handle, zeroed in the order of its stream (which
+    // does not wait for the default stream: a memset there could run after the
+    // first copy into the buffer).
     template <typename T>
     T *dalloc(size_t n) {
+        T *p = raw_alloc<T>(n);
+        DALM_CUDA(cudaMemsetAsync(p, 0, std::max<size_t>(n, 1) * sizeof(T), stream));
+        return p;
+    }
+    template <typename T>
+    T *raw_alloc(size_t n) {
         void *p = nullptr;
         DALM_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
-        DALM_CUDA(cudaMemset(p, 0, std::max<size_t>(n, 1) * sizeof(T)));
         allocs.push_back(p);
         return (T *)p;
     }
     template <typename T>
     T *upload(const std::vector<T> &v) {
-        T *p = dalloc<T>(v.size());
+        T *p = raw_alloc<T>(v.size());
         if (!v.empty())
-            DALM_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+            DALM_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
         return p;
     }
 
@@ -366,10 +374,7 @@ struct dalm_handle {
                     U32[b][m] = dalloc<float>(n);
                     JU32[b][m] = dalloc<float>(n);
                 }
-            for (int m = 0; m < 3; m++) {
-                F32[m] = dalloc<float>(n);
-                DALM_CUDA(cudaMemset(F32[m], 0, sizeof(float) * n));
-            }
+            for (int m = 0; m < 3; m++) F32[m] = dalloc<float>(n);
         }
         if (mixed) {
             float **kv32[] = {&pbf.x, &pbf.r, &pbf.r0, &pbf.pk, &pbf.q, &pbf.s, &pbf.t,
@@ -406,7 +411,7 @@ struct dalm_handle {
         memset(h_diag, 0, sizeof(DiagState));
         DiagState d0{};
         d0.ncell = (double)g.ni() * g.nj() * g.nk();
-        DALM_CUDA(cudaMemcpy(d_diag, &d0, sizeof(d0), cudaMemcpyHostToDevice));
+        DALM_CUDA(cudaMemcpyAsync(d_diag, &d0, sizeof(d0), cudaMemcpyHostToDevice, stream));
 
         P.g = g;
         P.m = mesh;
@@ -435,8 +440,9 @@ struct dalm_handle {
             std::vector<double> u((size_t)g.total);
             for (int m = 0; m < 3; m++) {
                 for (size_t c = 0; c < u.size(); c++) u[c] = (1. - solid_host[c]) * cs.uin[m];
-                DALM_CUDA(cudaMemcpy(U[ucur][m], u.data(), sizeof(double) * u.size(),
-                                     cudaMemcpyHostToDevice));
+                DALM_CUDA(cudaMemcpyAsync(U[ucur][m], u.data(), sizeof(double) * u.size(),
+                                          cudaMemcpyHostToDevice, stream));
+                DALM_CUDA(cudaStreamSynchronize(stream));
             }
         }
         narrow_state(false);
@@ -1929,8 +1935,9 @@ int dalm_set_inflow_profile(dalm_handle *h, const double *prof) {
         h->P.prof = nullptr;
     } else {
         if (!h->d_prof) h->d_prof = h->dalloc<double>((size_t)3 * h->g.ny * h->g.nz);
-        DALM_CUDA(cudaMemcpy(h->d_prof, prof, sizeof(double) * 3 * h->g.ny * h->g.nz,
-                             cudaMemcpyHostToDevice));
+        DALM_CUDA(cudaMemcpyAsync(h->d_prof, prof, sizeof(double) * 3 * h->g.ny * h->g.nz,
+                                  cudaMemcpyHostToDevice, h->stream));
+        DALM_CUDA(cudaStreamSynchronize(h->stream));
         h->P.prof = h->d_prof;
     }
     API_END(h)
@@ -1955,10 +1962,11 @@ int dalm_set_turbine_params(dalm_handle *h, const double *yaw_deg, const double 
             for (int a = w * per; a < (w + 1) * per; a++) h->twist[a] = h->base_twist[a] + pitch_deg[w];
         }
     }
-    DALM_CUDA(cudaMemcpy((void *)h->alm.wt, h->h_wt.data(), sizeof(TurbineDev) * T,
-                         cudaMemcpyHostToDevice));
-    DALM_CUDA(cudaMemcpy((void *)h->alm.twist, h->twist.data(), sizeof(double) * h->twist.size(),
-                         cudaMemcpyHostToDevice));
+    DALM_CUDA(cudaMemcpyAsync((void *)h->alm.wt, h->h_wt.data(), sizeof(TurbineDev) * T,
+                              cudaMemcpyHostToDevice, h->stream));
+    DALM_CUDA(cudaMemcpyAsync((void *)h->alm.twist, h->twist.data(), sizeof(double) * h->twist.size(),
+                              cudaMemcpyHostToDevice, h->stream));
+    DALM_CUDA(cudaStreamSynchronize(h->stream));
     API_END(h)
 }
 
