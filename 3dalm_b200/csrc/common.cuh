@@ -291,6 +291,20 @@ struct LaunchCtx {
     }
 };
 
+// Asynchronous copy of one double from global to shared memory (a
+// shared-window address); zeros are written instead when `in` is false.  The
+// thread's copies complete in the order of their commit groups.
+__device__ __forceinline__ void cp_async8(unsigned dst, const double *src, bool in) {
+    const int n = in ? 8 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Programmatic dependent launch: a kernel launched by pdl_launch may be
 // scheduled while the previous kernel in the stream is finishing, so its
 // launch latency overlaps that kernel's tail.  pdl_wait(), the first

@@ -322,9 +322,11 @@ struct dalm_handle {
                 std::vector<float4> t(x.size(), make_float4(0.f, 0.f, 0.f, 0.f));
                 std::vector<float2> w(x.size());
                 std::vector<double2> r(x.size(), make_double2(0.0, 0.0));
+                std::vector<double> id(x.size());
                 for (size_t n = 0; n < x.size(); n++) {
                     const double cb = std::cbrt(d[n]);
                     w[n] = make_float2((float)d[n], (float)(cb * cb));
+                    id[n] = 1.0 / d[n];
                     if (n + 1 < x.size()) r[n].x = 1.0 / (x[n + 1] - x[n]);
                     if (n >= 1 && n + 1 < x.size()) r[n].y = 1.0 / (x[n + 1] - x[n - 1]);
                 }
@@ -335,6 +337,8 @@ struct dalm_handle {
                 geo.ax[a] = upload(t);
                 geo.wd[a] = upload(w);
                 geo.inv64[a] = upload(r);
+                P.inv[a] = geo.inv64[a];
+                P.invd[a] = upload(id);
             }
             geo.cs2 = (float)(cs.cs * cs.cs);
         }

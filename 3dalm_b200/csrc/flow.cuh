@@ -37,6 +37,10 @@ struct StepParams {
     double uin[3];
     const double *prof;  // inflow profile [ny][nz][3] on the device, or null
     Box fbox;            // cells where the ALM force may be non-zero
+    // correctly rounded reciprocals per axis, for stored index n: inv
+    // {1/(x_{n+1} - x_n), 1/(x_{n+1} - x_{n-1})}, invd 1/d_n
+    const double2 *inv[3];
+    const double *invd[3];
     // (Cs * cbrt(dx dy dz))^2 per interior cell, computed once on the host
     // with the same libm cbrt the reference calls (src/cfd.h:804, 823-824)
     const double *filter2;
