@@ -121,7 +121,6 @@ struct dalm_handle {
     bool f32 = false;
     bool f64_stale = false;
     float *U32[2][3] = {}, *JU32[2][3] = {}, *F32[3] = {};
-    FusedBufs fb{};
     bool fused = false;  // BiCGStab iterations as fused half-iteration kernels
     PoissonConfig pcfg{};
     MapTable maps;
@@ -366,8 +365,9 @@ struct dalm_handle {
         pcfg.pc_sweeps = (int)cs.pc_max_it;
         pcfg.reference_sums = opt.reference_sums ? 1 : 0;
         pcfg.jacobi2 = opt.fused_jacobi ? 1 : 0;
+        pcfg.sm_count = sm_count;
         pcfg.seg = poisson_segments(g, sm_count);
-        fused = opt.fused_krylov && fused_bicg_available(pcfg);
+        choose_route();
         // FP32 inner solves exist for BiCGStab only; SOR and Jacobi solves
         // stay FP64 under DALM_MIXED
         mixed = opt.precision == DALM_MIXED && pcfg.method == PM_BICG;
@@ -387,18 +387,9 @@ struct dalm_handle {
             pbf.b = pbf.r0;  // e starts at 0, so the inner r0 = r = b
             if (opt.mixed_inner == DALM_INNER_MULTIGRID) setup_multigrid();
         }
-        fb = FusedBufs{{pb.pk, nullptr}, {pb.q, nullptr}};
-        if (fused) {
-            fb.pk[1] = dalloc<double>(n);
-            fb.q[1] = dalloc<double>(n);
-        }
         const double *tma_fields[] = {pb.x, pb.b, pb.r, pb.r0, pb.pk, pb.q,
                                       pb.s, pb.t, pb.pp, pb.ss, pb.tp, pb.ts};
         for (const double *v : tma_fields) maps.add(g, v);
-        if (fused) {
-            maps.add(g, fb.pk[1]);
-            maps.add(g, fb.q[1]);
-        }
         if (mixed) {
             const float *tma32[] = {pbf.x, pbf.r, pbf.r0, pbf.pk, pbf.q, pbf.s,
                                     pbf.t, pbf.pp, pbf.ss, pbf.tp, pbf.ts};
@@ -453,6 +444,14 @@ struct dalm_handle {
         refresh_after_state(DALM_SET_APPLY_UBC | DALM_SET_RECOMPUTE_JU, nullptr);
         DALM_CUDA(cudaStreamSynchronize(stream));
         if (opt.write_output) init_output();
+    }
+
+    // Jacobi(3)-BiCGStab runs as fused half-iterations on grids above 600 k
+    // cells (us per iteration, kernel per loop / fused: 192x96x64 125 / 107,
+    // 512x256x128 860 / 680; below, launches bound both: 128x64x64 84 / 75).
+    void choose_route() {
+        const long long cells = (long long)g.ni() * g.nj() * g.nk();
+        fused = fused_bicg_available(pcfg) && !opt.fused_jacobi && (opt.fused_krylov || cells > 600000);
     }
 
     // The multigrid levels of the inner solves (multigrid.cuh): merged-cell
@@ -718,7 +717,7 @@ struct dalm_handle {
     // iteration n (from 0) of the current solve
     void enqueue_poisson_iteration(long long n) {
         if (fused) {
-            launch_bicg_iteration_fused(L, g, coef, pb, fb, n, pcfg, Partials<2>{partial, ticket}, d_kst);
+            launch_bicg_iteration_fused(L, g, coef, pb, n, pcfg, Partials<2>{partial, ticket}, d_kst);
         } else if (pcfg.method == PM_BICG) {
             launch_bicg_iteration<double>(L, g, coef, pb, pcfg, Partials<2>{partial, ticket}, d_kst);
         } else if (pcfg.method == PM_SOR) {
@@ -731,7 +730,7 @@ struct dalm_handle {
         DALM_CUDA(cudaMemcpyAsync(h_kst, d_kst, 2 * sizeof(KrylovState), cudaMemcpyDeviceToHost, stream));
         DALM_CUDA(cudaStreamSynchronize(stream));
         if (h_kst[0].wait_error || h_kst[1].wait_error)
-            throw DeviceWaitError("a TMA stage wait in the Poisson solver ran out");
+            throw DeviceWaitError("a bounded wait in the Poisson solver ran out");
     }
     // Enqueues iterations of solve `which` in batches and polls the device's
     // `done` flag in between.  The first batch stops a little short of

@@ -66,6 +66,7 @@ struct PoissonConfig {
     int pc_sweeps;
     int reference_sums;  // 1: global sums in the reference's serial order
     int jacobi2;         // 1: FP64 Jacobi(3): the last two sweeps in one pass
+    int sm_count;
     Segments seg;        // column segments of the interior (one per block)
     const MapTable *maps;
 };
@@ -113,18 +114,15 @@ void launch_bicg_xr(const LaunchCtx &L, const Grid &g, const PoissonBufs &B, con
                     const double *ssf, const PoissonConfig &cfg, Partials<2> part,
                     KrylovState *st);
 
-// Ping-pong partners of p and q for the fused iteration: iteration n reads
-// pk[n % 2], q[n % 2] and writes pk[(n + 1) % 2], q[(n + 1) % 2].
-struct FusedBufs {
-    double *pk[2], *q[2];
-};
 // true when the fused kernels implement this configuration: BiCGStab with
 // 3 Jacobi sweeps, tree sums (not the reference-order mode)
 bool fused_bicg_available(const PoissonConfig &cfg);
 // BiCGStab iteration n (from 0) as two fused half-iteration kernels + the
-// x / r update (poisson_fused.cu)
+// x / r update (poisson_fused.cu).  p and q alternate between B.pk, B.q (read
+// by even iterations) and B.tp, B.ts.
 void launch_bicg_iteration_fused(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
-                                 const PoissonBufs &B, const FusedBufs &F, long long n,
-                                 const PoissonConfig &cfg, Partials<2> part, KrylovState *st);
+                                 const PoissonBufs &B, long long n, const PoissonConfig &cfg,
+                                 Partials<2> part, KrylovState *st);
+
 
 }  // namespace dalm

@@ -1,11 +1,11 @@
 // TMA (cp.async.bulk.tensor) plane staging for the stencil kernels.
 //
 // A field is described to the TMA unit as a 3-D tensor {x = k + off (the
-// padded row), y = j, z = i}.  Three maps per field: `halo` boxes of
+// padded row), y = j, z = i}.  Four maps per field: `halo` boxes of
 // (32 + 2h) x 10 x 1 elements (the 32 x 8 tile of a block plus one cell in
 // j and h cells in k each side, h = 16 B / element size so that the box
-// starts on a 16-byte boundary), `plain` boxes of 32 x 8 x 1 and `wide`
-// boxes (below).  Loads complete on an mbarrier per ring stage.  Every wait
+// starts on a 16-byte boundary), `plain` boxes of 32 x 8 x 1, `wide` and
+// `half` boxes (below).  Loads complete on an mbarrier per ring stage.  Every wait
 // is bounded: after WAIT_LIMIT polls the kernel raises an error flag and
 // returns.
 #pragma once
@@ -16,18 +16,23 @@
 
 namespace dalm {
 
-// `wide` boxes carry the three-cell halo of the fused BiCGStab kernels:
-// (32 + 2*4) x (8 + 2*3) x 1, starting 4 cells below the tile in k (a
-// 16-byte boundary for 4- and 8-byte elements) and 3 rows below it in j.
+// `wide` boxes carry the halo of the fused Jacobi pair: (32 + 2*4) x
+// (8 + 2*3) x 1, starting 4 cells below the tile in k (a 16-byte boundary for
+// 4- and 8-byte elements) and 3 rows below it in j.
 constexpr int WIDE_HK = 4, WIDE_HJ = 3;
+
+// `half` boxes of the BiCGStab half-iterations (poisson_half.cuh): W x ROWS
+// cells, for grids above or up to 32 cells high
+constexpr int WIDE_BOX_K = 72, WIDE_BOX_J = 21, NARROW_BOX_K = 40, NARROW_BOX_J = 24;
 
 struct FieldMaps {
     CUtensorMap halo;
     CUtensorMap plain;
     CUtensorMap wide;
+    CUtensorMap half;
 };
 
-// Builds both maps for one field (element size 4 or 8) over grid g; throws
+// Builds the maps of one field (element size 4 or 8) over grid g; throws
 // CudaError when the driver rejects them.
 FieldMaps make_field_maps(const Grid &g, const void *base, int elem_bytes);
 
@@ -48,6 +53,12 @@ __device__ __forceinline__ void fence_barrier_init() {
 
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// orders this thread's global writes (and those it has acquired) with
+// TMA loads of the same memory
+__device__ __forceinline__ void fence_proxy_global() {
+    asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
