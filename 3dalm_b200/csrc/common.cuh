@@ -263,6 +263,8 @@ enum KernelKind {
     KK_MG_SMOOTH, KK_MG_TRANSFER, KK_MG_COARSE, KK_MG_PCG,
     // two FP64 Jacobi sweeps in one pass (the preconditioner's last two)
     KK_JACOBI_SWEEP2,
+    // a small grid's whole FP64 solve (poisson_resident.cu)
+    KK_RESIDENT,
     KK_COUNT
 };
 

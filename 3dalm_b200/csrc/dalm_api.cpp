@@ -51,6 +51,9 @@ constexpr double INNER_RTOL = 1e-4;
 constexpr long long INNER_CAP = 100;
 constexpr double STALL = 0.85;
 constexpr long long MAX_REFINE = 1000;
+// Iterations per launch of a resident solve: bounds a launch to a fraction of a
+// second.
+constexpr long long RESIDENT_BUDGET = 1000;
 // Adjoint pressure solves stop at this RMS residual relative to the RMS of
 // their right-hand side.
 constexpr double ADJ_RTOL = 1e-10;
@@ -64,7 +67,7 @@ const char *kKindNames[KK_COUNT] = {
     "refine_update", "sor_sweep32", "jacobi_sweep32", "bicg_p32", "bicg_q32", "bicg_s32",
     "bicg_t32", "bicg_xr32", "adj_velocity_bc", "adj_project", "adj_faces", "adj_nut",
     "adj_predict", "adj_alm", "mg_smooth", "mg_transfer", "mg_coarse", "mg_pcg",
-    "jacobi_sweep2"};
+    "jacobi_sweep2", "resident_solve"};
 
 }  // namespace
 
@@ -121,7 +124,9 @@ struct dalm_handle {
     bool f32 = false;
     bool f64_stale = false;
     float *U32[2][3] = {}, *JU32[2][3] = {}, *F32[3] = {};
-    bool fused = false;  // BiCGStab iterations as fused half-iteration kernels
+    bool fused = false;     // BiCGStab iterations as fused half-iteration kernels
+    bool resident = false;  // whole FP64 solves as one cooperative kernel (choose_route)
+    unsigned *d_sync = nullptr;
     PoissonConfig pcfg{};
     MapTable maps;
     double *partial = nullptr;
@@ -398,6 +403,7 @@ struct dalm_handle {
         pcfg.maps = &maps;
         partial = dalloc<double>((size_t)std::max(L.blocks, pcfg.seg.count) * 4);
         ticket = dalloc<unsigned int>(1);
+        if (resident) d_sync = dalloc<unsigned int>(2);
         d_kst = dalloc<KrylovState>(2);  // [0] the solve (refinement: outer), [1] inner
         d_diag = dalloc<DiagState>(1);
         DALM_CUDA(cudaHostAlloc((void **)&h_kst, 2 * sizeof(KrylovState), cudaHostAllocDefault));
@@ -446,12 +452,23 @@ struct dalm_handle {
         if (opt.write_output) init_output();
     }
 
-    // Jacobi(3)-BiCGStab runs as fused half-iterations on grids above 600 k
-    // cells (us per iteration, kernel per loop / fused: 192x96x64 125 / 107,
-    // 512x256x128 860 / 680; below, launches bound both: 128x64x64 84 / 75).
+    // How an FP64 solve runs.  Whole, as one cooperative kernel, when that
+    // holds the grid (poisson_resident.cu: any SOR, Jacobi and SOR-preconditioned
+    // solve up to about 10 M cells, Jacobi(3)-BiCGStab up to eight cells a
+    // thread, 606,208 on 148 SMs): measured faster than a kernel per loop at
+    // every such size (us per iteration, launched / resident: SOR 26.3 / 7.3 on
+    // 128x64x64, 164 / 113 on 384x192x100; Jacobi 118 / 75 there; BiCGStab
+    // 74 / 29 on 100x40x33, 93 / 58 on 131x75x53).  Larger Jacobi(3)-BiCGStab
+    // solves run as fused half-iterations (192x96x64: 125 / 107, 512x256x128:
+    // 860 / 680).  fused_krylov and fused_jacobi ask for a launched form, and
+    // profiling times launches, so it keeps the kernel-per-loop form of small
+    // grids.
     void choose_route() {
-        const long long cells = (long long)g.ni() * g.nj() * g.nk();
-        fused = fused_bicg_available(pcfg) && !opt.fused_jacobi && (opt.fused_krylov || cells > 600000);
+        int coop = 0;
+        DALM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, opt.device));
+        const bool holds = coop && resident_available(pcfg, g);
+        fused = fused_bicg_available(pcfg) && !opt.fused_jacobi && (opt.fused_krylov || !holds);
+        resident = holds && !opt.fused_krylov && !opt.fused_jacobi && !opt.profile;
     }
 
     // The multigrid levels of the inner solves (multigrid.cuh): merged-cell
@@ -815,6 +832,15 @@ struct dalm_handle {
         }
         return h_kst[which].it;
     }
+    // the same loop for a resident solve: returns its iterations
+    long long run_resident(long long cap) {
+        for (long long issued = 0;; issued += RESIDENT_BUDGET) {
+            if (issued > cap) throw std::runtime_error("Poisson loop did not stop at its iteration limit");
+            launch_resident_solve(L, g, coef, pb, pcfg, RESIDENT_BUDGET, partial, d_sync, d_kst);
+            fetch_states();
+            if (h_kst[0].done) return h_kst[0].it;
+        }
+    }
     // The reference's solve (FP64) from the current p; `used` iterations of
     // the case's cap are already spent.
     void solve_fp64(long long used) {
@@ -823,7 +849,7 @@ struct dalm_handle {
         if (pcfg.method == PM_BICG)
             launch_bicg_init(L, g, coef, pb, pcfg, Partials<1>{partial, ticket}, d_kst);
         long long hint = mixed ? refine_fp64_it : last_it;
-        long long n = run_batches(0, hint, max_it - used);
+        long long n = resident ? run_resident(max_it - used) : run_batches(0, hint, max_it - used);
         refine_fp64_it = n;
         h_kst[0].it = used + n;
     }
@@ -1558,7 +1584,7 @@ struct dalm_handle {
         launch_poisson_begin(L, d_kst, max_it, tol_abs, ncell);
         if (pcfg.method == PM_BICG)
             launch_bicg_init(L, g, coef, pb, pcfg, Partials<1>{partial, ticket}, d_kst);
-        long long n = run_batches(0, adj_hint > 0 ? adj_hint : last_it, max_it);
+        long long n = resident ? run_resident(max_it) : run_batches(0, adj_hint > 0 ? adj_hint : last_it, max_it);
         adj_hint = n;
         return n;
     }

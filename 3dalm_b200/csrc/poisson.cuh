@@ -125,4 +125,15 @@ void launch_bicg_iteration_fused(const LaunchCtx &L, const Grid &g, const Poisso
                                  Partials<2> part, KrylovState *st);
 
 
+// true when a small grid's FP64 solve can run as one cooperative kernel
+// (poisson_resident.cu): SOR, Jacobi, BiCGStab with the Jacobi(3) or the SOR
+// preconditioner, not in the reference-order mode
+bool resident_available(const PoissonConfig &cfg, const Grid &g);
+// Up to `budget` iterations of the solve that launch_poisson_begin (and
+// launch_bicg_init) set up, or of the one an earlier launch left unfinished.
+// part: four doubles of device memory per SM; sync: two words.
+void launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
+                           const PoissonBufs &B, const PoissonConfig &cfg, long long budget,
+                           double *part, unsigned *sync, KrylovState *st);
+
 }  // namespace dalm

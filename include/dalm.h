@@ -135,12 +135,12 @@ typedef struct {
                              included (slow: for parity checks)          */
     int fused_krylov;     /* 1: each half of a Jacobi(3)-BiCGStab
                              iteration (update, preconditioner, SpMV, dot
-                             products) as one kernel, 20 instead of 35
-                             vectors per cell per iteration; 0 (default):
-                             one kernel per reference loop, which is as
-                             fast on B200 today (the fused kernels are
-                             latency-bound).  Ignored with reference_sums
-                             and other preconditioners.                 */
+                             products) as one kernel at every grid size, 20
+                             instead of 35 vectors per cell per iteration;
+                             0 (default): so on large grids, and a whole
+                             solve as one kernel on grids that fit the
+                             device's registers.  Ignored with
+                             reference_sums and other preconditioners.   */
     int refine_inner_it;  /* DALM_MIXED: FP32 iterations per refinement
                              pass before the FP64 residual is recomputed
                              (0: automatic, 100)                         */
@@ -151,12 +151,11 @@ typedef struct {
                              and a per-turbine turbines.csv every step   */
     int mixed_inner;      /* DALM_MIXED: the FP32 inner solver of each
                              refinement pass, enum dalm_mixed_inner      */
-    int fused_jacobi;     /* 1: the FP64 Jacobi(3) preconditioner's last
-                             two sweeps in one pass over HBM (3 instead of
-                             6 vectors per cell; same results bit for
-                             bit); 0 (default): one kernel per sweep,
-                             which is as fast under the power cap (the
-                             fused pair is instruction-bound)            */
+    int fused_jacobi;     /* 1: one kernel per loop of the reference, with
+                             the FP64 Jacobi(3) preconditioner's last two
+                             sweeps in one pass over HBM (3 instead of 6
+                             vectors per cell; the same results bit for
+                             bit as one kernel per sweep)                */
     int reserved[2];
 } dalm_options;
 
