@@ -51,6 +51,8 @@ constexpr double INNER_RTOL = 1e-4;
 constexpr long long INNER_CAP = 100;
 constexpr double STALL = 0.85;
 constexpr long long MAX_REFINE = 1000;
+// Largest grid whose coarse multigrid levels run as a cluster kernel.
+constexpr long long MG_CLUSTER_CELLS = 4000000;
 // Iterations per launch of a resident solve: bounds a launch to a fraction of a
 // second.
 constexpr long long RESIDENT_BUDGET = 1000;
@@ -493,9 +495,11 @@ struct dalm_handle {
             return;
         }
         mgd.levels = (int)geo.size();
+        std::vector<MgLevelHost> host((size_t)mgd.levels);
         for (int l = 0; l < mgd.levels; l++) {
             const MgGeometry &G = geo[l];
             MgLevel &v = mgd.L[l];
+            MgLevelHost &h = host[(size_t)l];
             v.g = l == 0 ? g : Grid::make(G.n[0] + 2, G.n[1] + 2, G.n[2] + 2, 1);
             std::vector<float> fcf[3], fw[3];
             for (int a = 0; a < 3; a++) {
@@ -505,12 +509,17 @@ struct dalm_handle {
                 fw[a].assign(G.w[a].begin(), G.w[a].end());
                 v.cf[a] = upload(fcf[a]);
                 v.w[a] = upload(fw[a]);
+                h.n[a] = G.n[a];
+                h.fac[a] = G.fac[a];
+                h.cf[a] = fcf[a];
+                h.w[a] = fw[a];
             }
             // the smoother's z-line factors on the two finest levels, when the
             // mesh allows (on the coarser, latency-bound levels the table's
             // loads cost more than the elimination they save: measured on C4)
-            MgLineTable T;
+            MgLineTable &T = h.table;
             if (l < 2 && mg_line_table(v.n, fcf, fw, T)) {
+                h.has_table = true;
                 v.lcls[0] = upload(T.cls[0]);
                 v.lcls[1] = upload(T.cls[1]);
                 v.lky = T.ky;
@@ -528,9 +537,32 @@ struct dalm_handle {
         std::vector<double> inv = mg_spd_inverse(mg_dense_operator(C), C.cells());
         mgd.kinv = upload(std::vector<float>(inv.begin(), inv.end()));
         mgd.ncoarse = (int)C.cells();
+        setup_mg_cluster(host);
         const size_t n = (size_t)g.total;
         mgb = MgPcgBufs{pbf.r, pbf.x, dalloc<float>(n), dalloc<float>(n), dalloc<float>(n)};
         mg_on = true;
+    }
+
+    // The levels that one cluster of blocks holds run as one kernel
+    // (multigrid_cluster.cu), from the first level that fits (ms per step,
+    // launches / cluster: 64x32x40 1.31 / 1.01, 160x96x72 3.30 / 2.91).  On
+    // large grids those levels are a few percent of a step (512x256x128 4.39 /
+    // 4.34), and the launches stay.  Profiling times the half-sweeps' launches
+    // and keeps them.
+    void setup_mg_cluster(const std::vector<MgLevelHost> &host) {
+        if (opt.profile || mgd.L[0].cells() > MG_CLUSTER_CELLS) return;
+        for (int first = 0; first + 1 < mgd.levels; first++) {
+            MgCluster M;
+            std::vector<float> image;
+            for (int blocks : {16, 8}) {  // 16: beyond the portable size, where the device takes it
+                M.top = mgd.L[first];
+                if (!mg_cluster_layout(host, first, blocks, MG_CLUSTER_WARPS, 220 * 1024, M, image) || !mg_cluster_fits(M)) continue;
+                M.kinv = mgd.kinv;
+                M.image = upload(image);
+                mgd.cluster = M;
+                return;
+            }
+        }
     }
 
     // Solid volume fraction of the turbulence-generating grid per interior

@@ -247,8 +247,33 @@ void mg_vcycle(E &e, int levels, int nu) {
 constexpr int MG_NU = 2;
 DALM_HD int mg_nu(int level) { return level == 0 ? 4 : level == 1 ? 3 : MG_NU; }
 
+// A level of the cluster V-cycle (multigrid_cluster.cu): sizes, and offsets in
+// 32-bit words into every block's shared memory.  x and f hold the block's
+// planes as [plane][n1][S], a column padded with zeros to S = 32 R rows.
+struct MgClusterLevel {
+    int n[3], fac[3];
+    int S;
+    int x, f;
+    int w0, cf0, w1, cf1, w2, cf2;  // widths and conductances (w2 padded with zeros to S)
+    int tab, cls, lky;              // factor table (-1: none) and its class numbers
+    int gather;                     // coarsest level: room for the whole f
+    int planes;                     // [n[0]] addresses of the planes of x, wherever they are
+};
+constexpr int MG_CLUSTER_WARPS = 16;  // per block
+// The levels from `first` on, for one cluster of `blocks` blocks.
+struct MgCluster {
+    int first = 0, levels = 0;  // levels 0: not used
+    int blocks = 0;
+    int words = 0, total = 0;   // words of the image, and of shared memory per block
+    int ncoarse = 0;
+    MgLevel top;                // level `first`, as it is in global memory
+    const float *image = nullptr;  // level table, coefficients, factor tables
+    const float *kinv = nullptr;
+};
+
 // Device state of the preconditioner (multigrid.cu).
 struct MgDev {
+    MgCluster cluster;
     int levels = 0;
     MgLevel L[MG_MAX_LEVELS];
     float *x[MG_MAX_LEVELS] = {}, *f[MG_MAX_LEVELS] = {};  // level 0: the caller's z and r
@@ -261,6 +286,12 @@ struct KrylovState;
 // False when the levels' z-columns are longer than the line smoother takes
 // (256 cells); the mixed form then keeps its BiCGStab inner solves.
 bool mg_prepare(const MgDev &M);
+
+// false when no cluster of this size and shared memory fits the device
+bool mg_cluster_fits(const MgCluster &M);
+// x of level M.first = the V-cycle from that level on, of its f
+void launch_mg_cluster(const LaunchCtx &L, const MgCluster &M, const float *f, float *x,
+                       const KrylovState *st);
 
 // x[0] = V-cycle(f[0]); every kernel returns at once when st->done is set.
 void launch_mg_vcycle(const LaunchCtx &L, const MgDev &M, const KrylovState *st);

@@ -5,6 +5,7 @@
 
 #include <array>
 #include <cmath>
+#include <cstring>
 #include <stdexcept>
 #include <vector>
 
@@ -258,6 +259,85 @@ inline bool mg_line_table(const int (&n)[3], const std::vector<float> (&cf)[3],
             for (int l = 0; l < 32; l++) put(mglf_invrb(R), l, 1.0 / rb[l]);
         }
     return true;
+}
+
+// FP32 coefficients of one level for the cluster V-cycle.
+struct MgLevelHost {
+    int n[3], fac[3];
+    std::vector<float> cf[3], w[3];
+    bool has_table = false;
+    MgLineTable table;
+};
+
+// Lays out the levels from `first` on for `blocks` blocks: fills M (but its
+// device pointers and `top`) and the image; false when they need more than
+// `limit` bytes of shared memory per block, columns above 128 cells, or more
+// than `warps` columns per block and half-sweep on the first level.
+inline bool mg_cluster_layout(const std::vector<MgLevelHost> &L, int first, int blocks, int warps, size_t limit,
+                              MgCluster &M, std::vector<float> &image) {
+    const int nl = (int)L.size() - first;
+    if (nl < 2) return false;
+    auto up4 = [](size_t n) { return (n + 3) / 4 * 4; };
+    std::vector<MgClusterLevel> lv((size_t)nl);
+    image.assign(up4(nl * sizeof(MgClusterLevel) / 4), 0.f);
+    auto add = [&](const float *v, size_t n, size_t padded) {
+        const size_t at = image.size();
+        image.insert(image.end(), v, v + n);
+        image.resize(at + up4(padded), 0.f);
+        return (int)at;
+    };
+    for (int m = 0; m < nl; m++) {
+        const MgLevelHost &h = L[(size_t)(first + m)];
+        MgClusterLevel &c = lv[(size_t)m];
+        for (int a = 0; a < 3; a++) {
+            c.n[a] = h.n[a];
+            c.fac[a] = h.fac[a];
+        }
+        if (h.n[2] > 128) return false;
+        c.S = (h.n[2] + 31) / 32 * 32;
+        c.w0 = add(h.w[0].data(), h.w[0].size(), h.w[0].size());
+        c.cf0 = add(h.cf[0].data(), h.cf[0].size(), h.cf[0].size());
+        c.w1 = add(h.w[1].data(), h.w[1].size(), h.w[1].size());
+        c.cf1 = add(h.cf[1].data(), h.cf[1].size(), h.cf[1].size());
+        c.w2 = add(h.w[2].data(), h.w[2].size(), (size_t)c.S);
+        c.cf2 = add(h.cf[2].data(), h.cf[2].size(), (size_t)c.S + 1);
+        c.tab = c.cls = -1;
+        c.lky = 0;
+        c.gather = c.planes = 0;
+        if (h.has_table) {
+            c.lky = h.table.ky;
+            c.tab = add(h.table.tab.data(), h.table.tab.size(), h.table.tab.size());
+            std::vector<float> cls((size_t)(h.n[0] + h.n[1]));
+            for (int i = 0; i < h.n[0] + h.n[1]; i++) {
+                const int v = i < h.n[0] ? h.table.cls[0][(size_t)i] : h.table.cls[1][(size_t)(i - h.n[0])];
+                std::memcpy(&cls[(size_t)i], &v, 4);
+            }
+            c.cls = add(cls.data(), cls.size(), cls.size());
+        }
+    }
+    M.first = first;
+    M.levels = nl;
+    M.blocks = blocks;
+    M.words = (int)image.size();
+    size_t at = image.size();
+    for (int m = 0; m < nl; m++) {
+        MgClusterLevel &c = lv[(size_t)m];
+        const size_t planes = (size_t)((c.n[0] + blocks - 1) / blocks);
+        if (planes * (size_t)((c.n[1] + 1) / 2) > (size_t)warps) return false;
+        c.x = (int)at;
+        at += planes * (size_t)c.n[1] * (size_t)c.S;
+        c.f = (int)at;
+        at += planes * (size_t)c.n[1] * (size_t)c.S;
+        c.planes = (int)at;
+        at += up4(2 * (size_t)c.n[0]);
+    }
+    const MgClusterLevel &last = lv.back();
+    M.ncoarse = last.n[0] * last.n[1] * last.n[2];
+    lv.back().gather = (int)at;
+    at += up4((size_t)M.ncoarse);
+    M.total = (int)at;
+    std::memcpy(image.data(), lv.data(), lv.size() * sizeof(MgClusterLevel));
+    return at * 4 <= limit;
 }
 
 }  // namespace dalm
