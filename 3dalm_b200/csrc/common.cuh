@@ -78,37 +78,8 @@ struct Box {
     }
 };
 
-// Tiling of a box into (32 k) x (8 j) x (1 i) tiles; blocks of 256 threads
-// walk the tiles with a block-stride loop so the number of blocks (and thus
-// the number of reduction partials) is fixed per launch.
+// Tiles of (32 k) x (8 j) cells, one cell per thread of a block.
 constexpr int TK = 32, TJ = 8, TILE_THREADS = TK * TJ;
-
-struct Tiling {
-    Box box;
-    int ntk, ntj, nti;
-    long long ntiles;
-    __host__ static Tiling make(const Box &b) {
-        Tiling t;
-        t.box = b;
-        t.ntk = (b.hi[2] - b.lo[2] + TK - 1) / TK;
-        t.ntj = (b.hi[1] - b.lo[1] + TJ - 1) / TJ;
-        t.nti = b.hi[0] - b.lo[0];
-        if (b.empty()) t.ntk = t.ntj = t.nti = 0;
-        t.ntiles = (long long)t.ntk * t.ntj * t.nti;
-        return t;
-    }
-    // cell handled by this thread in tile `tile`; false when outside the box
-    __device__ bool cell(long long tile, int &i, int &j, int &k) const {
-        int tk = (int)(tile % ntk);
-        long long r = tile / ntk;
-        int tj = (int)(r % ntj);
-        int ti = (int)(r / ntj);
-        k = box.lo[2] + tk * TK + (int)(threadIdx.x % TK);
-        j = box.lo[1] + tj * TJ + (int)(threadIdx.x / TK);
-        i = box.lo[0] + ti;
-        return k < box.hi[2] && j < box.hi[1];
-    }
-};
 
 // Column segments: the box is cut into (32 k) x (8 j) columns, and each
 // column into i-chunks of `ich` planes.  One block of 256 threads owns one
@@ -251,7 +222,7 @@ __device__ inline bool grid_reduce(double (&v)[N], unsigned maxmask, Partials<N>
 // Kinds of kernels, for launch counting and per-kernel event timing.
 enum KernelKind {
     KK_PREDICT = 0, KK_FLUX_RHS, KK_PBC, KK_PROJECT, KK_UBC, KK_DIAG, KK_TAVG,
-    KK_ALM_POINTS, KK_ALM_SUMS, KK_ALM_PROJECT,
+    KK_ALM_POINTS, KK_ALM_PROJECT,
     KK_SOR_SWEEP, KK_RESIDUAL_NORM, KK_JACOBI_SWEEP,
     KK_BICG_INIT, KK_BICG_P, KK_BICG_Q, KK_BICG_S, KK_BICG_T, KK_BICG_XR,
     KK_POISSON_BEGIN, KK_LAYOUT, KK_SEQ_SUM, KK_BICG_PF, KK_BICG_SF, KK_REFINE_RESIDUAL, KK_REFINE_UPDATE,

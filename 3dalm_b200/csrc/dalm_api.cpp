@@ -62,7 +62,7 @@ constexpr double ADJ_RTOL = 1e-10;
 
 const char *kKindNames[KK_COUNT] = {
     "predict", "flux_rhs", "pressure_bc", "project", "velocity_bc", "diag", "tavg",
-    "alm_points", "alm_sums", "alm_project",
+    "alm_points", "alm_project",
     "sor_sweep", "residual_norm", "jacobi_sweep",
     "bicg_init", "bicg_p", "bicg_q", "bicg_s", "bicg_t", "bicg_xr",
     "poisson_begin", "layout", "seq_sum", "bicg_p_fused", "bicg_s_fused", "refine_residual",
