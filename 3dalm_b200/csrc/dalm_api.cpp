@@ -129,6 +129,7 @@ struct dalm_handle {
     bool fused = false;     // BiCGStab iterations as fused half-iteration kernels
     bool resident = false;  // whole FP64 solves as one cooperative kernel (choose_route)
     unsigned *d_sync = nullptr;
+    bool states_ahead = false;  // the last solve's state is on the device only
     PoissonConfig pcfg{};
     MapTable maps;
     double *partial = nullptr;
@@ -778,8 +779,18 @@ struct dalm_handle {
     void fetch_states() {
         DALM_CUDA(cudaMemcpyAsync(h_kst, d_kst, 2 * sizeof(KrylovState), cudaMemcpyDeviceToHost, stream));
         DALM_CUDA(cudaStreamSynchronize(stream));
-        if (h_kst[0].wait_error || h_kst[1].wait_error)
-            throw DeviceWaitError("a bounded wait in the Poisson solver ran out");
+        states_ahead = false;
+        check_waits();
+    }
+    // A bounded device wait that ran out stays marked in the state over later
+    // solves until it is reported here.
+    void check_waits() {
+        if (!h_kst[0].wait_error && !h_kst[1].wait_error) return;
+        for (int q = 0; q < 2; q++) {
+            h_kst[q].wait_error = 0;
+            DALM_CUDA(cudaMemsetAsync(&d_kst[q].wait_error, 0, sizeof(int), stream));
+        }
+        throw DeviceWaitError("a bounded wait in the Poisson solver ran out");
     }
     // Enqueues iterations of solve `which` in batches and polls the device's
     // `done` flag in between.  The first batch stops a little short of
@@ -880,6 +891,13 @@ struct dalm_handle {
         launch_poisson_begin(L, d_kst, max_it - used, tol, ncell);
         if (pcfg.method == PM_BICG)
             launch_bicg_init(L, g, coef, pb, pcfg, Partials<1>{partial, ticket}, d_kst);
+        // a resident solve that ends within one launch needs no answer here:
+        // the step goes on, and its statistics come with the next ones read
+        states_ahead = resident && !mixed && !trace && max_it - used <= RESIDENT_BUDGET;
+        if (states_ahead) {
+            launch_resident_solve(L, g, coef, pb, pcfg, RESIDENT_BUDGET, partial, d_sync, d_kst);
+            return;
+        }
         long long hint = mixed ? refine_fp64_it : last_it;
         long long n = resident ? run_resident(max_it - used) : run_batches(0, hint, max_it - used);
         refine_fp64_it = n;
@@ -1842,10 +1860,13 @@ struct dalm_handle {
         if (J_out) *J_out = J;
     }
 
-    // The last step's diagnostics and turbine loads into their pinned host
-    // copies, enqueued where a reader is about to synchronise rather than
-    // every step (each small copy costs the stream a few microseconds).
+    // The last step's diagnostics, turbine loads and, when the solve was not
+    // waited for, its state into their pinned host copies, enqueued where a
+    // reader is about to synchronise rather than every step (each small copy
+    // costs the stream a few microseconds).
     void fetch_step_outputs() {
+        if (states_ahead)
+            DALM_CUDA(cudaMemcpyAsync(h_kst, d_kst, sizeof(KrylovState), cudaMemcpyDeviceToHost, stream));
         DALM_CUDA(cudaMemcpyAsync(h_diag, d_diag, sizeof(DiagState), cudaMemcpyDeviceToHost, stream));
         if (alm.ap_count > 0) {
             DALM_CUDA(cudaMemcpyAsync(h_wt_out, alm.wt_torque, sizeof(double) * alm.wt_count,
@@ -1857,6 +1878,11 @@ struct dalm_handle {
     void sync_stats() {
         fetch_step_outputs();
         DALM_CUDA(cudaStreamSynchronize(stream));
+        if (states_ahead) {
+            states_ahead = false;
+            last_it = h_kst[0].it;
+            check_waits();
+        }
         if (opt.profile) harvest();
     }
 };
