@@ -168,72 +168,83 @@ __device__ __forceinline__ bool zline_column(const MgLevel &L, unsigned col, uns
     return j < L.n[1];
 }
 
-template <int R>
-__device__ __forceinline__ void zline_load(const MgLevel &L, const float *x, const float *f, int i,
-                                           int j, int lane, ColumnLoads<R> &v) {
-    const long long c0 = L.at(i, j, 0) + R * lane;
-    load_seg<R>(f + c0, v.f);
-    load_seg<R>(x + c0 + L.g.sx, v.e);
-    load_seg<R>(x + c0 - L.g.sx, v.w);
-    load_seg<R>(x + c0 + L.g.sy, v.n);
-    load_seg<R>(x + c0 - L.g.sy, v.s);
-}
+// A column's widths and conductances along x and y.
+struct ColumnCoef {
+    float wi, wj, xe, xw, yn, ys;
+    __device__ __forceinline__ void load(const MgLevel &L, int i, int j) {
+        wi = L.w[0][i], wj = L.w[1][j];
+        xe = L.cf[0][i + 1], xw = L.cf[0][i], yn = L.cf[1][j + 1], ys = L.cf[1][j];
+    }
+};
 
 // The VEC half-sweep without a pending prolongation (all but the first
-// half-sweep after a coarse correction), software-pipelined over the
-// columns a warp takes: the next column's operands are loaded before the
-// current column is solved, so their latency overlaps the line solve.  Same
-// arithmetic as k_mg_smooth's VEC path.
+// half-sweep after a coarse correction); the grid is what fits the device at
+// once, smooth_blocks(R) blocks per SM.  FAC: the columns of one class have
+// the same line factors and neighbour coefficients, so a warp keeps them in
+// registers and reads them again only where the class changes (on a uniform
+// mesh: at the grid's edges).
+//
+// Bound by issue and latency.  With the factors (26 loads at R = 4) and the
+// coefficients read for every column it took 292 instructions a column, and
+// 512x256x128 4.35 ms a step; this form 4.00 ms.  Prefetching the next
+// column's operands costs the registers of a third block (4.31 ms), four
+// blocks per SM spill (4.26 ms).
+constexpr int smooth_blocks(int R) { return R <= 4 ? 3 : 2; }
 template <int R, bool FAC>
-__global__ void __launch_bounds__(MG_THREADS) k_mg_smooth_pipe(ZlineArgs A, const KrylovState *st) {
+__global__ void __launch_bounds__(MG_THREADS, smooth_blocks(R)) k_mg_smooth_rows(ZlineArgs A, const KrylovState *st) {
     pdl_wait();
     if (st->done) return;
     const MgLevel &L = A.L;
     float *__restrict__ x = A.x;
     const float *__restrict__ f = A.f;
-    const int lane = threadIdx.x & 31;
-    const unsigned njh = (unsigned)(L.n[1] + 1) / 2;
+    const int lane = threadIdx.x & 31, nj = L.n[1];
+    const unsigned njh = (unsigned)(nj + 1) / 2;
     const unsigned ncol = (unsigned)L.n[0] * njh;
     const unsigned nw = gridDim.x * (blockDim.x >> 5);
-    const int nk = L.n[2];
     const bool zero = A.zero_start != 0;
-    const float *w2 = L.w[2], *cf2 = L.cf[2];
-    float vw2[R];
-    load_seg<R>(w2 + R * lane, vw2);
+    const int sx = (int)L.g.sx, sy = (int)L.g.sy, base = (int)L.at(0, 0, 0) + R * lane;
+    float w2[R];
+    load_seg<R>(L.w[2] + R * lane, w2);
     unsigned col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    int i = 0, j = 0;
-    bool ok = col < ncol && zline_column(L, col, njh, A.color, i, j);
-    ColumnLoads<R> cur, nxt;
-    if (ok) zline_load<R>(L, x, f, i, j, lane, cur);
-    while (col < ncol) {
-        const unsigned ncol2 = col + nw;
-        int i2 = 0, j2 = 0;
-        const bool ok2 = ncol2 < ncol && zline_column(L, ncol2, njh, A.color, i2, j2);
-        if (ok2) zline_load<R>(L, x, f, i2, j2, lane, nxt);
-        if (ok) {
-            const float wi = L.w[0][i], wj = L.w[1][j];
-            const float xe = L.cf[0][i + 1], xw = L.cf[0][i], yn = L.cf[1][j + 1], ys = L.cf[1][j];
-            float d[R], xs[R];
-#pragma unroll
-            for (int q = 0; q < R; q++)
-                d[q] = zero ? cur.f[q]
-                            : cur.f[q] + vw2[q] * (wj * (xe * cur.e[q] + xw * cur.w[q]) +
-                                                   wi * (yn * cur.n[q] + ys * cur.s[q]));
-            if (FAC) {
-                line_solve_table<R>(L.ltab + (size_t)(L.lcls[0][i] * L.lky + L.lcls[1][j]) *
-                                                 mglf_count(R) * 32 + lane,
-                                    lane, d, xs);
-            } else {
-                const float az = wi * wj, sxy = wj * (xe + xw) + wi * (yn + ys);
-                line_solve<R>(az, sxy, w2, cf2, nk, lane, d, xs);
-            }
-            store_seg<R>(x + L.at(i, j, 0) + R * lane, xs);
+    Stepper pos(col, nw, njh);
+    LineFactors<R> F;
+    ColumnCoef K;
+    int cls = -1;
+    for (; col < ncol; col += nw, pos.next()) {
+        const int i = (int)pos.i, j = 2 * (int)pos.h + ((i + A.color) & 1);
+        if (j >= nj) continue;  // uniform in the warp
+        const int c = base + i * sx + j * sy;
+        ColumnLoads<R> v;
+        load_seg<R>(f + c, v.f);
+        if (!zero) {
+            load_seg<R>(x + (c + sx), v.e);
+            load_seg<R>(x + (c - sx), v.w);
+            load_seg<R>(x + (c + sy), v.n);
+            load_seg<R>(x + (c - sy), v.s);
         }
-        col = ncol2;
-        i = i2;
-        j = j2;
-        ok = ok2;
-        cur = nxt;
+        float d[R], xs[R];
+        if (FAC) {
+            const int q = L.lcls[0][i] * L.lky + L.lcls[1][j];
+            if (q != cls) {
+                cls = q;
+                F.load(L.ltab + (size_t)q * mglf_count(R) * 32 + lane);
+                K.load(L, i, j);
+            }
+        } else {
+            K.load(L, i, j);
+        }
+#pragma unroll
+        for (int q = 0; q < R; q++)
+            d[q] = zero ? v.f[q]
+                        : v.f[q] + w2[q] * (K.wj * (K.xe * v.e[q] + K.xw * v.w[q]) +
+                                            K.wi * (K.yn * v.n[q] + K.ys * v.s[q]));
+        if (FAC) {
+            F.solve(lane, d, xs);
+        } else {
+            const float az = K.wi * K.wj, sxy = K.wj * (K.xe + K.xw) + K.wi * (K.yn + K.ys);
+            line_solve<R>(az, sxy, L.w[2], L.cf[2], L.n[2], lane, d, xs);
+        }
+        store_seg<R>(x + c, xs);
     }
 }
 
@@ -388,18 +399,21 @@ bool zline_vec_ok(const ZlineArgs &a, int R) {
 template <int R>
 void zline_launch(const LaunchCtx &L, const ZlineArgs &a, const KrylovState *st, int blocks) {
     const bool vec = zline_vec_ok(a, R);
-    if (vec && !a.xc && a.L.ltab)
-        pdl_launch(k_mg_smooth_pipe<R, true>, blocks, MG_THREADS, 0, L.s, a, st);
-    else if (vec && !a.xc)
-        pdl_launch(k_mg_smooth_pipe<R, false>, blocks, MG_THREADS, 0, L.s, a, st);
-    else if (a.L.ltab && vec)
-        pdl_launch(k_mg_smooth<R, true, true>, blocks, MG_THREADS, 0, L.s, a, st);
-    else if (a.L.ltab)
-        pdl_launch(k_mg_smooth<R, true, false>, blocks, MG_THREADS, 0, L.s, a, st);
-    else if (vec)
-        pdl_launch(k_mg_smooth<R, false, true>, blocks, MG_THREADS, 0, L.s, a, st);
-    else
-        pdl_launch(k_mg_smooth<R, false, false>, blocks, MG_THREADS, 0, L.s, a, st);
+    if constexpr (R == 1 || R == 2 || R == 4 || R == 8) {
+        if (vec && !a.xc) {
+            const int fit = std::min(blocks, L.blocks / 8 * smooth_blocks(R));  // L.blocks: 8 per SM
+            if (a.L.ltab) pdl_launch(k_mg_smooth_rows<R, true>, fit, MG_THREADS, 0, L.s, a, st);
+            else pdl_launch(k_mg_smooth_rows<R, false>, fit, MG_THREADS, 0, L.s, a, st);
+            return;
+        }
+        if (vec) {
+            if (a.L.ltab) pdl_launch(k_mg_smooth<R, true, true>, blocks, MG_THREADS, 0, L.s, a, st);
+            else pdl_launch(k_mg_smooth<R, false, true>, blocks, MG_THREADS, 0, L.s, a, st);
+            return;
+        }
+    }
+    if (a.L.ltab) pdl_launch(k_mg_smooth<R, true, false>, blocks, MG_THREADS, 0, L.s, a, st);
+    else pdl_launch(k_mg_smooth<R, false, false>, blocks, MG_THREADS, 0, L.s, a, st);
 }
 
 void zline_dispatch(const LaunchCtx &L, const ZlineArgs &a, const KrylovState *st) {
