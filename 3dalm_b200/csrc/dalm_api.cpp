@@ -519,8 +519,11 @@ struct dalm_handle {
             // mesh allows (on the coarser, latency-bound levels the table's
             // loads cost more than the elimination they save: measured on C4)
             MgLineTable &T = h.table;
-            if (l < 2 && mg_line_table(v.n, fcf, fw, T)) {
-                h.has_table = true;
+            // The cluster's warps read them once per visit, for several
+            // half-sweeps, and have them on every level.
+            const bool cluster = !opt.profile && geo[0].cells() <= MG_CLUSTER_CELLS;
+            h.has_table = (l < 2 || cluster) && mg_line_table(v.n, fcf, fw, T);
+            if (l < 2 && h.has_table) {
                 v.lcls[0] = upload(T.cls[0]);
                 v.lcls[1] = upload(T.cls[1]);
                 v.lky = T.ky;
@@ -546,7 +549,7 @@ struct dalm_handle {
 
     // The levels that one cluster of blocks holds run as one kernel
     // (multigrid_cluster.cu), from the first level that fits (ms per step,
-    // launches / cluster: 64x32x40 1.31 / 1.01, 160x96x72 3.30 / 2.91).  On
+    // launches / cluster: 64x32x40 1.31 / 0.90, 160x96x72 3.30 / 2.70).  On
     // large grids those levels are a few percent of a step (512x256x128 4.39 /
     // 4.34), and the launches stay.  Profiling times the half-sweeps' launches
     // and keeps them.
@@ -554,12 +557,13 @@ struct dalm_handle {
         if (opt.profile || mgd.L[0].cells() > MG_CLUSTER_CELLS) return;
         for (int first = 0; first + 1 < mgd.levels; first++) {
             MgCluster M;
-            std::vector<float> image;
+            std::vector<float> image, tables;
             for (int blocks : {16, 8}) {  // 16: beyond the portable size, where the device takes it
                 M.top = mgd.L[first];
-                if (!mg_cluster_layout(host, first, blocks, MG_CLUSTER_WARPS, 220 * 1024, M, image) || !mg_cluster_fits(M)) continue;
+                if (!mg_cluster_layout(host, first, blocks, MG_CLUSTER_WARPS, 220 * 1024, M, image, tables) || !mg_cluster_fits(M)) continue;
                 M.kinv = mgd.kinv;
                 M.image = upload(image);
+                M.tables = tables.empty() ? nullptr : upload(tables);
                 mgd.cluster = M;
                 return;
             }

@@ -255,7 +255,7 @@ struct MgClusterLevel {
     int S;
     int x, f;
     int w0, cf0, w1, cf1, w2, cf2;  // widths and conductances (w2 padded with zeros to S)
-    int tab, cls, lky;              // factor table (-1: none) and its class numbers
+    int tab, cls, lky;              // factor table in MgCluster::tables (-1: none), its class numbers
     int gather;                     // coarsest level: room for the whole f
     int planes;                     // [n[0]] addresses of the planes of x, wherever they are
 };
@@ -266,8 +266,10 @@ struct MgCluster {
     int blocks = 0;
     int words = 0, total = 0;   // words of the image, and of shared memory per block
     int ncoarse = 0;
+    int zeros = 0;              // a column of zeros
     MgLevel top;                // level `first`, as it is in global memory
-    const float *image = nullptr;  // level table, coefficients, factor tables
+    const float *image = nullptr;   // level table and coefficients
+    const float *tables = nullptr;  // line factors (MgLevel::ltab) of the levels that have them
     const float *kinv = nullptr;
 };
 

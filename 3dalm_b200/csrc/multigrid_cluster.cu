@@ -11,11 +11,17 @@
 // its x goes back.
 //
 // What bounds it: the chain of a half-sweep, neighbour loads, line solve, store
-// and barrier.  A block's warps take at most one column each per half-sweep, so
-// levels with more columns than the cluster has warps stay launches over the
-// whole device (with four columns a warp on the first level the kernel was
-// slower than the launches it replaced).  64x32x40: 50 us for the 34 phases of
-// four levels, against about 2.7 us for each of the launches.
+// and barrier, at about ten cycles an instruction.  A block's warps take at
+// most one column each per half-sweep, so levels with more columns than the
+// cluster has warps stay launches over the whole device (with four columns a
+// warp on the first level the kernel was slower than the launches it replaced).
+// So what a visit can do once is done once, before its half-sweeps: the line's
+// factors come from the tables, addresses and coefficients stay in registers,
+// and what lies past the grid is a column of zeros instead of a branch.
+// 64x32x40 took 0.98 ms a step with factors eliminated in each visit, generic
+// addresses and a spilled state, now 0.90; 160x96x72 2.89, now 2.70.  Small
+// levels whole in one block, with block barriers for cluster barriers, gained
+// nothing.
 //
 // Operations are mg_vcycle's in the folded form of DeviceCycle (multigrid.cu):
 // the restriction leaves out the colour smoothed last, and a prolongation is
@@ -41,20 +47,47 @@ __device__ __forceinline__ unsigned cluster_rank() {
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-// the same shared-memory address in block `rank` of the cluster
-__device__ __forceinline__ const float *in_block(const float *p, unsigned rank) {
-    const float *r;
-    asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+__device__ __forceinline__ void copy_async(float *shared, const float *global) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(shared)),
+                 "l"(global)
+                 : "memory");
+}
+// the address of a word of shared memory in block `rank` of the cluster
+__device__ __forceinline__ unsigned in_block(const float *p, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
     return r;
+}
+// loads and a store at such an address.  Volatile: they keep their place
+// between the cluster barriers.
+__device__ __forceinline__ float load_word(unsigned a) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void store_word(unsigned a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+template <int R>
+__device__ __forceinline__ void load_rows(unsigned a, float (&v)[R]) {
+    if constexpr (R == 4)
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                     : "r"(a));
+    else if constexpr (R == 2)
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(a));
+    else
+#pragma unroll
+        for (int t = 0; t < R; t++) v[t] = load_word(a + 4 * t);
 }
 
 // A level as a block sees it.
 struct Lv {
     const MgClusterLevel *c;
     float *x, *f;             // this block's planes
-    const float **planes;     // every plane of x, in the block that owns it
-    int to_f;                 // from a column of x to the same column of f
-    const float *w0, *cf0, *w1, *cf1, *w2, *cf2, *tab;
+    const unsigned *planes;   // every plane of x, in the block that owns it
+    int to_f;                 // bytes from a column of x to the same column of f
+    const float *w0, *cf0, *w1, *cf1, *w2, *cf2;
     const int *cls0, *cls1;
 };
 
@@ -65,28 +98,30 @@ struct Cycle {
     unsigned rank, blocks;
     float *sm;
     const MgClusterLevel *lv;  // in shared memory
+    const float *tables;       // line factors, in global memory
+    float *zeros;              // a column of zeros: what lies past the grid
+    unsigned zeros_at;
     int lane, warp;
 
     // planes [first(r), first(r + 1)) of a level belong to block r
-    __device__ __forceinline__ int first(int ni, unsigned r) const {
-        return (int)((r * (unsigned)ni + blocks - 1) / blocks);
+    __device__ __forceinline__ int first(const MgClusterLevel &c, unsigned r) const {
+        return (int)((r * (unsigned)c.n[0] + blocks - 1) / blocks);
     }
     __device__ __forceinline__ Lv level(int l) const {
         const MgClusterLevel &c = lv[l];
         const int *cls = reinterpret_cast<const int *>(sm) + c.cls;
-        return Lv{&c, sm + c.x, sm + c.f, reinterpret_cast<const float **>(sm + c.planes), c.f - c.x,
-                  sm + c.w0, sm + c.cf0, sm + c.w1, sm + c.cf1, sm + c.w2, sm + c.cf2, sm + c.tab,
+        return Lv{&c, sm + c.x, sm + c.f, reinterpret_cast<const unsigned *>(sm + c.planes), 4 * (c.f - c.x),
+                  sm + c.w0, sm + c.cf0, sm + c.w1, sm + c.cf1, sm + c.w2, sm + c.cf2,
                   cls, cls + c.n[0]};
     }
     // the addresses of every level's planes
     __device__ __forceinline__ void map_planes(int levels) const {
         for (int l = 0; l < levels; l++) {
             const MgClusterLevel &c = lv[l];
-            const float **planes = reinterpret_cast<const float **>(sm + c.planes);
+            unsigned *planes = reinterpret_cast<unsigned *>(sm + c.planes);
             for (int i = threadIdx.x; i < c.n[0]; i += CT) {
                 const unsigned o = (unsigned)i * blocks / (unsigned)c.n[0];
-                const float *p = sm + c.x + (i - first(c.n[0], o)) * c.n[1] * c.S;
-                planes[i] = o == rank ? p : in_block(p, o);
+                planes[i] = in_block(sm + c.x + (i - first(c, o)) * c.n[1] * c.S, o);
             }
         }
     }
@@ -102,77 +137,77 @@ struct Cycle {
     __device__ __forceinline__ void visit(int l, int nu, bool post) const {
         const Lv L = level(l);
         const MgClusterLevel &c = *L.c;
-        const int i0 = first(c.n[0], rank), np = first(c.n[0], rank + 1) - i0;
+        const int i0 = first(c, rank), np = first(c, rank + 1) - i0;
         const int n0 = c.n[0], n1 = c.n[1], S = c.S, njh = (n1 + 1) / 2;
         const int ip = warp / njh, h = warp - ip * njh, i = i0 + ip;
-        const bool in = ip < np;  // uniform in the warp, as everything but the lane
+        if (ip >= np) {  // no column: only the barriers (uniform in the warp, as all but the lane)
+            for (int s = 0; s < 2 * nu; s++) cluster_sync();
+            return;
+        }
         LineFactors<R> F[2];
-        float f[2][R], w2[R], wj[2], yn[2], ys[2];
-        int at[2];
+        float f[2][R], w2[R], ke[2], kw[2], kn[2], ks[2];
+        unsigned e[2], w[2];               // the neighbours' rows of this lane
+        const float *nn[2], *ss[2];
+        float *at[2];
         bool has[2];
-        const float wi = in ? L.w0[i] : 0.f, xe = in ? L.cf0[i + 1] : 0.f, xw = in ? L.cf0[i] : 0.f;
         load_seg<R>(L.w2 + R * lane, w2);
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            const int j = 2 * h + ((i + q) & 1);
-            has[q] = in && j < n1;
-            at[q] = (ip * n1 + j) * S + R * lane;
-            if (!has[q]) continue;
-            wj[q] = L.w1[j], yn[q] = L.cf1[j + 1], ys[q] = L.cf1[j];
-            load_seg<R>(L.f + at[q], f[q]);
+            const int jq = 2 * h + ((i + q) & 1), j = min(jq, n1 - 1), col = j * S + R * lane;
+            has[q] = jq < n1;  // (an odd count's last: solved with the others, not stored)
+            const float wi = L.w0[i], xe = L.cf0[i + 1], xw = L.cf0[i];
+            const float wj = L.w1[j], yn = L.cf1[j + 1], ys = L.cf1[j];
+            ke[q] = wj * xe, kw[q] = wj * xw, kn[q] = wi * yn, ks[q] = wi * ys;
+            at[q] = L.x + ip * n1 * S + col;
+            e[q] = i + 1 < n0 ? L.planes[i + 1] + 4 * col : zeros_at;
+            w[q] = i > 0 ? L.planes[i - 1] + 4 * col : zeros_at;
+            nn[q] = j + 1 < n1 ? at[q] + S : zeros;
+            ss[q] = j > 0 ? at[q] - S : zeros;
+            load_seg<R>(at[q] + (c.f - c.x), f[q]);
             if (c.tab >= 0)
-                F[q].load(L.tab + (L.cls0[i] * c.lky + L.cls1[j]) * mglf_count(R) * 32 + lane);
+                F[q].load(tables + c.tab + (L.cls0[i] * c.lky + L.cls1[j]) * mglf_count(R) * 32 + lane);
             else
-                F[q].factor(wi * wj[q], wj[q] * (xe + xw) + wi * (yn[q] + ys[q]), L.w2, L.cf2, c.n[2], lane);
+                F[q].factor(wi * wj, wj * (xe + xw) + wi * (yn + ys), L.w2, L.cf2, c.n[2], lane);
         }
-        const float *east = in && i + 1 < n0 ? L.planes[i + 1] : nullptr;
-        const float *west = in && i > 0 ? L.planes[i - 1] : nullptr;
         auto half = [&](auto colour, bool zero, bool pending) {
             constexpr int q = decltype(colour)::value;  // constant: the arrays stay in registers
-            if (has[q]) {
-                const int j = 2 * h + ((i + q) & 1);
-                float d[R], x[R];
+            float d[R], x[R];
 #pragma unroll
-                for (int t = 0; t < R; t++) d[t] = f[q][t];
-                if (!zero) {
-                    float e[R], w[R], n[R], s[R];
-                    auto nb = [&](const float *p, int ii, int jj, float (&v)[R]) {
-                        if (!p) {
+            for (int t = 0; t < R; t++) d[t] = f[q][t];
+            if (!zero) {
+                float ve[R], vw[R], vn[R], vs[R];
+                load_rows<R>(e[q], ve);
+                load_rows<R>(w[q], vw);
+                load_seg<R>(nn[q], vn);
+                load_seg<R>(ss[q], vs);
+                if (pending) {
+                    // (a level merges one or two cells along an axis)
+                    const Lv C = level(l + 1);
+                    const int j = min(2 * h + ((i + q) & 1), n1 - 1), s0 = C.c->fac[0] - 1, s1 = C.c->fac[1] - 1;
+                    auto add = [&](bool there, int ii, int jj, float (&v)[R]) {
+                        if (!there) return;
+                        const unsigned xc = C.planes[ii >> s0] + 4 * (jj >> s1) * C.c->S;
 #pragma unroll
-                            for (int t = 0; t < R; t++) v[t] = 0.f;
-                            return;
-                        }
-                        load_seg<R>(p, v);
-                        if (pending) {
-                            const Lv C = level(l + 1);
-                            const float *xc = C.planes[ii / C.c->fac[0]] + jj / C.c->fac[1] * C.c->S;
-                            const int shift = C.c->fac[2] == 2 ? 1 : 0;
-#pragma unroll
-                            for (int t = 0; t < R; t++)
-                                if (R * lane + t < c.n[2]) v[t] += xc[(R * lane + t) >> shift];
-                        }
+                        for (int t = 0; t < R; t++) v[t] += load_word(xc + 4 * ((R * lane + t) >> (C.c->fac[2] - 1)));
                     };
-                    nb(east ? east + j * S + R * lane : nullptr, i + 1, j, e);
-                    nb(west ? west + j * S + R * lane : nullptr, i - 1, j, w);
-                    nb(j + 1 < n1 ? L.x + at[q] + S : nullptr, i, j + 1, n);
-                    nb(j > 0 ? L.x + at[q] - S : nullptr, i, j - 1, s);
-#pragma unroll
-                    for (int t = 0; t < R; t++)
-                        d[t] = d[t] + w2[t] * (wj[q] * (xe * e[t] + xw * w[t]) + wi * (yn[q] * n[t] + ys[q] * s[t]));
+                    add(i + 1 < n0, i + 1, j, ve);
+                    add(i > 0, i - 1, j, vw);
+                    add(j + 1 < n1, i, j + 1, vn);
+                    add(j > 0, i, j - 1, vs);
                 }
-                F[q].solve(lane, d, x);
-                store_seg<R>(L.x + at[q], x);
+#pragma unroll
+                for (int t = 0; t < R; t++)
+                    d[t] += w2[t] * (ke[q] * ve[t] + kw[q] * vw[t] + (kn[q] * vn[t] + ks[q] * vs[t]));
             }
+            F[q].solve(lane, d, x);
+            if (has[q]) store_seg<R>(at[q], x);
             cluster_sync();
         };
-        for (int s = 0; s < nu; s++) {
-            if (post) {
-                half(Colour<1>{}, false, s == 0);
-                half(Colour<0>{}, false, false);
-            } else {
-                half(Colour<0>{}, s == 0, false);
-                half(Colour<1>{}, false, false);
-            }
+#pragma unroll 1
+        for (int s = 0; s < 2 * nu; s++) {
+            const bool begin = s == 0;
+            if ((s & 1) == (post ? 1 : 0)) half(Colour<0>{}, begin, false);  // (begin: not after a correction)
+            else half(Colour<1>{}, false, begin);
         }
     }
     template <int RMAX>
@@ -184,64 +219,93 @@ struct Cycle {
         if (RMAX >= 4 && R == 4) visit<4>(l, nu, post);
     }
 
+    // A cell column's operands for its residual.
+    struct Child {
+        unsigned x, e, w, n, s;
+        float ce, cw, cn, cs, w0, w1, az, sxy;
+        __device__ __forceinline__ Child(const Lv &F, int i, int j, unsigned zeros_at) {
+            const MgClusterLevel &f = *F.c;
+            const unsigned row = 4u * (unsigned)f.S, col = j * row;
+            x = F.planes[i] + col;
+            e = i + 1 < f.n[0] ? F.planes[i + 1] + col : zeros_at;
+            w = i > 0 ? F.planes[i - 1] + col : zeros_at;
+            n = j + 1 < f.n[1] ? x + row : zeros_at;
+            s = j > 0 ? x - row : zeros_at;
+            w0 = F.w0[i], w1 = F.w1[j], az = w0 * w1;
+            ce = F.cf0[i + 1], cw = F.cf0[i], cn = F.cf1[j + 1], cs = F.cf1[j];
+            sxy = w1 * (ce + cw) + w0 * (cn + cs);
+        }
+        // f - K x at k
+        __device__ __forceinline__ float residual(const Lv &F, int k) const {
+            const unsigned o = 4u * (unsigned)k;
+            const float xk = load_word(x + o), rhs = load_word(x + F.to_f + o);
+            const float xe = load_word(e + o), xw = load_word(w + o), xn = load_word(n + o), xs = load_word(s + o);
+            const float xt = k + 1 < F.c->n[2] ? load_word(x + o + 4) : 0.f, xb = k > 0 ? load_word(x + o - 4) : 0.f;
+            const float w2 = F.w2[k], zt = F.cf2[k + 1], zb = F.cf2[k];
+            const float diag = w2 * sxy + az * (zt + zb);
+            const float nb = w2 * (w1 * (ce * xe + cw * xw) + w0 * (cn * xn + cs * xs)) + az * (zt * xt + zb * xb);
+            return rhs - (diag * xk - nb);
+        }
+    };
+
     // f of level l + 1: the sums of the children's residuals f - K x, the
-    // children of colour `skip` (whose residual is zero) left out
-    __device__ __forceinline__ void restrict_to(int l, int skip) const {
+    // children of colour 1 (smoothed last, no residual) left out: of two by
+    // two columns two are kept, of two one, of one one or none.
+    __device__ __forceinline__ void restrict_to(int l) const {
         const Lv F = level(l), C = level(l + 1);
-        const MgClusterLevel &f = *F.c, &c = *C.c;
-        const int I0 = first(c.n[0], rank), np = first(c.n[0], rank + 1) - I0, f2 = c.fac[2];
+        const MgClusterLevel &c = *C.c;
+        const int I0 = first(c, rank), np = first(c, rank + 1) - I0, fx = c.fac[0], fy = c.fac[1];
         for (int q = warp; q < np * c.n[1]; q += CW) {
-            const int ip = q / c.n[1], I = I0 + ip, J = q - ip * c.n[1];
-            float *out = C.f + (ip * c.n[1] + J) * c.S;
+            const int ip = q / c.n[1], I = I0 + ip, J = q - ip * c.n[1], i = I * fx, j = J * fy;
+            float *out = C.f + q * c.S;
+            // the kept column of the first row of children, then of the second
+            const int odd = (i + j) & 1;
+            const bool one = !odd || fy == 2, two = fx == 2 && (odd || fy == 2);
+            const Child A(F, one ? i : i + fx - 1, one ? j + odd : j, zeros_at);
+            const Child B(F, i + fx - 1, odd || fy == 1 ? j : j + 1, zeros_at);
+#pragma unroll 1
             for (int K = lane; K < c.n[2]; K += 32) {
                 float sum = 0.f;
-                for (int a = 0; a < c.fac[0]; a++)
-                    for (int b = 0; b < c.fac[1]; b++) {
-                        const int i = I * c.fac[0] + a, j = J * c.fac[1] + b;
-                        if (((i + j) & 1) == skip) continue;
-                        const float *x = F.planes[i] + j * f.S, *rhs = x + F.to_f;
-                        const float *xe = i + 1 < f.n[0] ? F.planes[i + 1] + j * f.S : nullptr;
-                        const float *xw = i > 0 ? F.planes[i - 1] + j * f.S : nullptr;
-                        const float *xn = j + 1 < f.n[1] ? x + f.S : nullptr, *xs = j > 0 ? x - f.S : nullptr;
-                        const float w0 = F.w0[i], w1 = F.w1[j], az = w0 * w1;
-                        const float ce = F.cf0[i + 1], cw = F.cf0[i], cn = F.cf1[j + 1], cs = F.cf1[j];
-                        const float sxy = w1 * (ce + cw) + w0 * (cn + cs);
-                        for (int t = 0; t < f2; t++) {
-                            const int k = K * f2 + t;
-                            const float w2 = F.w2[k], zt = F.cf2[k + 1], zb = F.cf2[k];
-                            const float diag = w2 * sxy + az * (zt + zb);
-                            const float nb =
-                                w2 * (w1 * (ce * (xe ? xe[k] : 0.f) + cw * (xw ? xw[k] : 0.f)) +
-                                      w0 * (cn * (xn ? xn[k] : 0.f) + cs * (xs ? xs[k] : 0.f))) +
-                                az * (zt * (k + 1 < f.n[2] ? x[k + 1] : 0.f) + zb * (k > 0 ? x[k - 1] : 0.f));
-                            sum += rhs[k] - (diag * x[k] - nb);
-                        }
-                    }
+#pragma unroll 1
+                for (int t = 0; t < c.fac[2]; t++) {
+                    const int k = K * c.fac[2] + t;
+                    const float ra = A.residual(F, k), rb = B.residual(F, k);
+                    sum += (one ? ra : 0.f) + (two ? rb : 0.f);
+                }
                 out[K] = sum;
             }
         }
         cluster_sync();
     }
 
-    // x = K^-1 f on the coarsest level: a warp per row of the dense inverse
+    // x = K^-1 f on the coarsest level: a warp per row of the dense inverse,
+    // the rows dealt out over all blocks
     __device__ __forceinline__ void coarse(int l, const float *kinv, int n) const {
         const Lv L = level(l);
         const MgClusterLevel &c = *L.c;
-        const int i0 = first(c.n[0], rank), np = first(c.n[0], rank + 1) - i0;
         float *all = sm + c.gather;  // the level's f in cell order
-        for (int r = threadIdx.x; r < n; r += CT) {
-            const int k = r % c.n[2], row = r / c.n[2], j = row % c.n[1], i = row / c.n[1];
-            all[r] = L.planes[i][j * c.S + L.to_f + k];
+        const int nk = c.n[2];
+        for (int col = warp; col < c.n[0] * c.n[1]; col += CW) {
+            const int i = col / c.n[1], j = col - i * c.n[1];
+            const unsigned f = L.planes[i] + 4 * j * c.S + L.to_f;
+            for (int k = lane; k < nk; k += 32) all[col * nk + k] = load_word(f + 4 * k);
         }
         __syncthreads();
-        const int plane = c.n[1] * c.n[2];
-        for (int q = warp; q < np * plane; q += CW) {
-            const float *row = kinv + (size_t)(i0 * plane + q) * n;
+        for (int q = (int)(rank + blocks * warp); q < n; q += (int)blocks * CW) {
+            const float *row = kinv + (size_t)q * n;
             float s = 0.f;
-            for (int r = lane; r < n; r += 32) s += row[r] * all[r];
+            for (int r0 = lane; r0 < n; r0 += MG_COARSE_TARGET) {
+                float v[MG_COARSE_TARGET / 32];
+#pragma unroll
+                for (int t = 0; t < MG_COARSE_TARGET / 32; t++) v[t] = r0 + 32 * t < n ? row[r0 + 32 * t] : 0.f;
+#pragma unroll
+                for (int t = 0; t < MG_COARSE_TARGET / 32; t++)
+                    if (r0 + 32 * t < n) s += v[t] * all[r0 + 32 * t];
+            }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-            if (lane == 0) L.x[q / c.n[2] * c.S + q % c.n[2]] = s;
+            const int k = q % nk, col = q / nk, i = col / c.n[1], j = col - i * c.n[1];
+            if (lane == 0) store_word(L.planes[i] + 4 * (j * c.S + k), s);
         }
         cluster_sync();
     }
@@ -251,12 +315,10 @@ struct Cycle {
 template <int RMAX>
 __global__ void __launch_bounds__(CT, 1)
 k_mg_cluster(MgCluster M, const float *f, float *x, const KrylovState *st) {
-    pdl_wait();
-    if (st->done) return;  // the same in every block
     extern __shared__ __align__(16) float cluster_smem[];
     float *sm = cluster_smem;
-    // the level table, its coefficients and factor tables; x and f zeroed (the
-    // lanes' rows past a column's end stay zero)
+    // the level table and its coefficients; x and f zeroed (the lanes' rows
+    // past a column's end stay zero)
     for (int n = threadIdx.x; n < M.words; n += CT) sm[n] = M.image[n];
     for (int n = M.words + threadIdx.x; n < M.total; n += CT) sm[n] = 0.f;
     __syncthreads();
@@ -265,24 +327,35 @@ k_mg_cluster(MgCluster M, const float *f, float *x, const KrylovState *st) {
     y.blocks = M.blocks;
     y.sm = sm;
     y.lv = reinterpret_cast<const MgClusterLevel *>(sm);
+    y.tables = M.tables;
+    y.zeros = sm + M.zeros;
+    y.zeros_at = in_block(y.zeros, y.rank);
     y.lane = threadIdx.x & 31;
     y.warp = threadIdx.x >> 5;
     y.map_planes(M.levels);
     const MgClusterLevel &c = y.lv[0];
-    const int i0 = y.first(c.n[0], y.rank), np = y.first(c.n[0], y.rank + 1) - i0;
+    const int i0 = y.first(c, y.rank), np = y.first(c, y.rank + 1) - i0;
+    pdl_wait();
+    if (st->done) return;  // the same in every block
     for (int q = y.warp; q < np * c.n[1]; q += CW) {
         const int ip = q / c.n[1], j = q - ip * c.n[1];
         const float *src = f + M.top.at(i0 + ip, j, 0);
-        for (int k = y.lane; k < c.n[2]; k += 32) sm[c.f + q * c.S + k] = src[k];
+        for (int k = y.lane; k < c.n[2]; k += 32) copy_async(sm + c.f + q * c.S + k, src + k);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     cluster_sync();
     const int last = M.levels - 1;
-    for (int l = 0; l < last; l++) {
-        y.smooth<RMAX>(l, mg_nu(M.first + l), false);
-        y.restrict_to(l, 1);
+    // down the levels, the coarsest solve, and up again
+#pragma unroll 1
+    for (int t = 0; t <= 2 * last; t++) {
+        if (t == last) {
+            y.coarse(last, M.kinv, M.ncoarse);
+            continue;
+        }
+        const int l = t < last ? t : 2 * last - t;
+        y.smooth<RMAX>(l, mg_nu(M.first + l), t > last);
+        if (t < last) y.restrict_to(l);
     }
-    y.coarse(last, M.kinv, M.ncoarse);
-    for (int l = last - 1; l >= 0; l--) y.smooth<RMAX>(l, mg_nu(M.first + l), true);
     for (int q = y.warp; q < np * c.n[1]; q += CW) {
         const int ip = q / c.n[1], j = q - ip * c.n[1];
         float *dst = x + M.top.at(i0 + ip, j, 0);

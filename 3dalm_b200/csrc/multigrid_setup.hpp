@@ -270,16 +270,17 @@ struct MgLevelHost {
 };
 
 // Lays out the levels from `first` on for `blocks` blocks: fills M (but its
-// device pointers and `top`) and the image; false when they need more than
+// device pointers and `top`), the image and the tables; false when they need more than
 // `limit` bytes of shared memory per block, columns above 128 cells, or more
 // than `warps` columns per block and half-sweep on the first level.
 inline bool mg_cluster_layout(const std::vector<MgLevelHost> &L, int first, int blocks, int warps, size_t limit,
-                              MgCluster &M, std::vector<float> &image) {
+                              MgCluster &M, std::vector<float> &image, std::vector<float> &tables) {
     const int nl = (int)L.size() - first;
     if (nl < 2) return false;
     auto up4 = [](size_t n) { return (n + 3) / 4 * 4; };
     std::vector<MgClusterLevel> lv((size_t)nl);
     image.assign(up4(nl * sizeof(MgClusterLevel) / 4), 0.f);
+    tables.clear();
     auto add = [&](const float *v, size_t n, size_t padded) {
         const size_t at = image.size();
         image.insert(image.end(), v, v + n);
@@ -306,7 +307,8 @@ inline bool mg_cluster_layout(const std::vector<MgLevelHost> &L, int first, int 
         c.gather = c.planes = 0;
         if (h.has_table) {
             c.lky = h.table.ky;
-            c.tab = add(h.table.tab.data(), h.table.tab.size(), h.table.tab.size());
+            c.tab = (int)tables.size();
+            tables.insert(tables.end(), h.table.tab.begin(), h.table.tab.end());
             std::vector<float> cls((size_t)(h.n[0] + h.n[1]));
             for (int i = 0; i < h.n[0] + h.n[1]; i++) {
                 const int v = i < h.n[0] ? h.table.cls[0][(size_t)i] : h.table.cls[1][(size_t)(i - h.n[0])];
@@ -329,12 +331,14 @@ inline bool mg_cluster_layout(const std::vector<MgLevelHost> &L, int first, int 
         c.f = (int)at;
         at += planes * (size_t)c.n[1] * (size_t)c.S;
         c.planes = (int)at;
-        at += up4(2 * (size_t)c.n[0]);
+        at += up4((size_t)c.n[0]);
     }
     const MgClusterLevel &last = lv.back();
     M.ncoarse = last.n[0] * last.n[1] * last.n[2];
     lv.back().gather = (int)at;
     at += up4((size_t)M.ncoarse);
+    M.zeros = (int)at;
+    at += (size_t)lv[0].S;
     M.total = (int)at;
     std::memcpy(image.data(), lv.data(), lv.size() * sizeof(MgClusterLevel));
     return at * 4 <= limit;
