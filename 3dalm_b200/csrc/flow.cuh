@@ -93,6 +93,57 @@ __device__ inline void warp_serial_sums(const Grid &g, Term term, double (&total
             }
 }
 
+// a / b with IEEE rounding, from y = 1 / b rounded to nearest (Markstein, IBM
+// J. Res. Dev. 34 (1990): with y the correctly rounded reciprocal and q
+// within one unit of a / b, q + (a - b q) y rounds to the correctly rounded
+// quotient; the first correction brings a y within one unit).  Five FP64
+// operations against the fourteen or so and the branch of a division.  b is a
+// mesh spacing or volume.  The remainders are exact for a = 0 and from
+// |a| = 2^-900 up; below that the quotient may be two units off, and an
+// infinite a gives NaN (the step reports either as a non-finite state).
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q0 = a * y;
+    const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+
+// The cells of the face box (the interior and one layer below it per axis)
+// outside the interior, n-th of face_shell_cells: the layer i = gc - 1, then
+// j = gc - 1, then k = gc - 1 of what is left.  The main kernels take the
+// interior alone, whose rows are aligned and a multiple of their tiles where
+// the face box, one cell longer, is neither (128 cells: five tiles of 32
+// along k instead of four, none on a sector boundary); extra blocks of the
+// same launch take these cells.
+__host__ __device__ inline long long face_shell_cells(const Grid &g) {
+    return (long long)(g.nj() + 1) * (g.nk() + 1) + (long long)g.ni() * (g.nk() + 1) +
+           (long long)g.ni() * g.nj();
+}
+__device__ __forceinline__ void face_shell_cell(const Grid &g, long long n, int &i, int &j, int &k) {
+    const int ni = g.ni(), nj = g.nj(), nk = g.nk(), lo = g.gc - 1;
+    i = j = k = lo;
+    if (n < (long long)(nj + 1) * (nk + 1)) {
+        j += (int)(n / (nk + 1));
+        k += (int)(n % (nk + 1));
+        return;
+    }
+    n -= (long long)(nj + 1) * (nk + 1);
+    if (n < (long long)ni * (nk + 1)) {
+        i += 1 + (int)(n / (nk + 1));
+        k += (int)(n % (nk + 1));
+        return;
+    }
+    n -= (long long)ni * (nk + 1);
+    i += 1 + (int)(n / nj);
+    j += 1 + (int)(n % nj);
+}
+
+// blocks for the faces below the interior: a few cells per thread, and no
+// more blocks than the reduction has partials for
+inline int shell_blocks(const Grid &g, const Segments &T) {
+    const long long b = (face_shell_cells(g) + 2 * TILE_THREADS - 1) / (2 * TILE_THREADS);
+    return (int)std::min<long long>(b, T.count);
+}
+
 // ---- flow kernels (flow_fp64.cu) ----
 void launch_predict(const LaunchCtx &L, const StepParams &P, Vec3<const double> uold,
                     Vec3<double> unew, Vec3<const double> ju, Vec3<const double> f);

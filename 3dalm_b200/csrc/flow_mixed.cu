@@ -299,6 +299,16 @@ __global__ void __launch_bounds__(256) k_copy_guides32(Grid g, Vec3<const float>
     }
 }
 
+// Mean volume flux through a face from the velocities below and above it.
+// The fused product is spelled out, so that a face has the same bits wherever
+// it is formed (x: the upper product, y and z: the lower one).
+__device__ __forceinline__ float mean_x32(float u0, float u1, float area) {
+    return 0.5f * __fmaf_rn(u1, area, __fmul_rn(u0, area));
+}
+__device__ __forceinline__ float mean_yz32(float u0, float u1, float area) {
+    return 0.5f * __fmaf_rn(u0, area, __fmul_rn(u1, area));
+}
+
 // Face flux with the apply_JUbc overrides (src/bc.h:235-302 and the inflow
 // profile extension); faces are named by their lower cell.  FP32.
 __device__ __forceinline__ float flux_x32(const StepParams &P, float u0, float u1, float yz, int i,
@@ -306,7 +316,7 @@ __device__ __forceinline__ float flux_x32(const StepParams &P, float u0, float u
     const Grid &g = P.g;
     if (i == g.gc - 1 && j >= g.gc && j < g.ny - g.gc && k >= g.gc && k < g.nz - g.gc)
         return yz * (float)(P.prof ? P.prof[((long long)j * g.nz + k) * 3] : P.uin[0]);
-    return 0.5f * (u0 * yz + u1 * yz);
+    return mean_x32(u0, u1, yz);
 }
 __device__ __forceinline__ float flux_y32(const StepParams &P, float v0, float v1, float xz, int i,
                                           int j, int k) {
@@ -314,7 +324,7 @@ __device__ __forceinline__ float flux_y32(const StepParams &P, float v0, float v
     if ((j == g.gc - 1 || j == g.ny - g.gc - 1) && i >= g.gc && i < g.nx - g.gc && k >= g.gc &&
         k < g.nz - g.gc)
         return 0.f;
-    return 0.5f * (v0 * xz + v1 * xz);
+    return mean_yz32(v0, v1, xz);
 }
 __device__ __forceinline__ float flux_z32(const StepParams &P, float w0, float w1, float xy, int i,
                                           int j, int k) {
@@ -322,71 +332,86 @@ __device__ __forceinline__ float flux_z32(const StepParams &P, float w0, float w
     if ((k == g.gc - 1 || k == g.nz - g.gc - 1) && i >= g.gc && i < g.nx - g.gc && j >= g.gc &&
         j < g.ny - g.gc)
         return 0.f;
-    return 0.5f * (w0 * xy + w1 * xy);
+    return mean_yz32(w0, w1, xy);
 }
 
 // Face fluxes on faces [gc-1, N-gc) per axis, and for RHS the Poisson
 // right-hand side b = div(JU) / (dt max_diag) of the interior cells in FP64
-// from the stored FP32 faces.  The west face of a cell is the previous
-// plane's east face (carried); the south and bottom faces are recomputed.
-// Software-pipelined along i: plane i + 1's velocities are loaded before
-// plane i is computed.
+// from the stored FP32 faces.  Blocks [0, T.count) march the interior's
+// column segments: the west face of a cell is the previous plane's east face
+// (carried), the south and bottom faces are recomputed, and plane i + 1's
+// velocities are loaded before plane i is computed.  The other blocks take
+// the faces below the interior (face_shell_cell).
+// Bound by memory latency and traffic.  512x256x128: 164 us, against 204 us
+// over the face box, whose rows of 129 cells take a fifth tile of 32 that is
+// nearly empty and start off the sector boundaries.
 struct FluxOps {
     float ue, v, vn, vs, w, wt, wb;  // U0 at i + 1; U1 at j, j + 1, j - 1; U2 at k, k + 1, k - 1
 };
 
-__device__ __forceinline__ void load_flux_ops(Vec3<const float> U, long long c, long long sx,
-                                              long long sy, bool rhs, FluxOps &o) {
+template <bool RHS>
+__device__ __forceinline__ void load_flux_ops(Vec3<const float> U, int c, int sx, int sy, FluxOps &o) {
     o.ue = U.c[0][c + sx];
     o.v = U.c[1][c];
     o.vn = U.c[1][c + sy];
     o.w = U.c[2][c];
     o.wt = U.c[2][c + 1];
-    o.vs = rhs ? U.c[1][c - sy] : 0.f;
-    o.wb = rhs ? U.c[2][c - 1] : 0.f;
+    o.vs = RHS ? U.c[1][c - sy] : 0.f;
+    o.wb = RHS ? U.c[2][c - 1] : 0.f;
 }
 
 template <bool RHS>
 __global__ void __launch_bounds__(TILE_THREADS)
 k_flux32(StepParams P, Segments T, MixedGeom Gm, Vec3<const float> U, Vec3<float> JU, double *b) {
     const Grid &g = P.g;
-    const long long sx = g.sx, sy = g.sy;
-    const double inv_dtm = 1.0 / (P.dt * P.max_diag);
-    for (int u = blockIdx.x; u < T.count; u += gridDim.x) {
-        int i0, i1, j, k;
-        if (!T.column(u, i0, i1, j, k)) continue;
-        const float dy = Gm.wd[1][j].x, dz = Gm.wd[2][k].x;
-        const double dyz64 = P.m.dy[j] * P.m.dz[k];
-        const float yz = dy * dz;
-        const bool jk_in = j >= g.gc && j < g.ny - g.gc && k >= g.gc && k < g.nz - g.gc;
-        long long c = g.at(i0, j, k);
-        float u_c = U.c[0][c];
-        float fw = 0.f;
-        if (RHS && i0 > g.gc - 1) fw = flux_x32(P, U.c[0][c - sx], u_c, yz, i0 - 1, j, k);
-        // rhs loads only where b is computed (interior j, k; any interior i)
-        FluxOps cur{}, nxt{};
-        load_flux_ops(U, c, sx, sy, RHS && jk_in, cur);
-        for (int i = i0; i < i1; i++, c += sx) {
-            if (i + 1 < i1) load_flux_ops(U, c + sx, sx, sy, RHS && jk_in, nxt);
-            const float dx = Gm.wd[0][i].x;
-            const float fe = flux_x32(P, u_c, cur.ue, yz, i, j, k);
-            const float fn = flux_y32(P, cur.v, cur.vn, dx * dz, i, j, k);
-            const float ft = flux_z32(P, cur.w, cur.wt, dx * dy, i, j, k);
-            JU.c[0][c] = fe;
-            JU.c[1][c] = fn;
-            JU.c[2][c] = ft;
-            if (RHS && jk_in && i >= g.gc && i < g.nx - g.gc) {
-                const float fs = flux_y32(P, cur.vs, cur.v, dx * dz, i, j - 1, k);
-                const float fb = flux_z32(P, cur.wb, cur.w, dx * dy, i, j, k - 1);
-                const double vol = P.m.dx[i] * dyz64;
-                const double div = ((double)fe - (double)fw + (double)fn - (double)fs +
-                                    (double)ft - (double)fb) / vol;
-                b[c] = div * inv_dtm;
-            }
-            fw = fe;
-            u_c = cur.ue;
-            cur = nxt;
+    const int sx = (int)g.sx, sy = (int)g.sy;
+    int i0, i1, j, k;
+    if ((int)blockIdx.x >= T.count) {
+        const long long step = (long long)(gridDim.x - T.count) * blockDim.x;
+        for (long long n = (long long)(blockIdx.x - T.count) * blockDim.x + threadIdx.x;
+             n < face_shell_cells(g); n += step) {
+            int i;
+            face_shell_cell(g, n, i, j, k);
+            const int c = (int)g.at(i, j, k);
+            const float dx = Gm.wd[0][i].x, dy = Gm.wd[1][j].x, dz = Gm.wd[2][k].x;
+            JU.c[0][c] = flux_x32(P, U.c[0][c], U.c[0][c + sx], dy * dz, i, j, k);
+            JU.c[1][c] = flux_y32(P, U.c[1][c], U.c[1][c + sy], dx * dz, i, j, k);
+            JU.c[2][c] = flux_z32(P, U.c[2][c], U.c[2][c + 1], dx * dy, i, j, k);
         }
+        return;
+    }
+    if (!T.column(blockIdx.x, i0, i1, j, k)) return;
+    const double inv_dtm = 1.0 / (P.dt * P.max_diag);
+    const float dy = Gm.wd[1][j].x, dz = Gm.wd[2][k].x;
+    const double dyz64 = P.m.dy[j] * P.m.dz[k];
+    const float yz = dy * dz;
+    const bool wall_n = j == g.ny - g.gc - 1, wall_s = j == g.gc;
+    const bool wall_t = k == g.nz - g.gc - 1, wall_b = k == g.gc;
+    int c = (int)g.at(i0, j, k);
+    float u_c = U.c[0][c];
+    float fw = RHS ? flux_x32(P, U.c[0][c - sx], u_c, yz, i0 - 1, j, k) : 0.f;
+    FluxOps cur, nxt;
+    load_flux_ops<RHS>(U, c, sx, sy, cur);
+    for (int i = i0; i < i1; i++, c += sx) {
+        if (i + 1 < i1) load_flux_ops<RHS>(U, c + sx, sx, sy, nxt);
+        const float dx = Gm.wd[0][i].x, xz = dx * dz, xy = dx * dy;
+        const float fe = mean_x32(u_c, cur.ue, yz);
+        const float fn = wall_n ? 0.f : mean_yz32(cur.v, cur.vn, xz);
+        const float ft = wall_t ? 0.f : mean_yz32(cur.w, cur.wt, xy);
+        JU.c[0][c] = fe;
+        JU.c[1][c] = fn;
+        JU.c[2][c] = ft;
+        if (RHS) {
+            const float fs = wall_s ? 0.f : mean_yz32(cur.vs, cur.v, xz);
+            const float fb = wall_b ? 0.f : mean_yz32(cur.wb, cur.w, xy);
+            const double vol = P.m.dx[i] * dyz64;
+            const double div = ((double)fe - (double)fw + (double)fn - (double)fs +
+                                (double)ft - (double)fb) / vol;
+            b[c] = div * inv_dtm;
+        }
+        fw = fe;
+        u_c = cur.ue;
+        cur = nxt;
     }
 }
 
@@ -395,106 +420,110 @@ k_flux32(StepParams P, Segments T, MixedGeom Gm, Vec3<const float> U, Vec3<float
 // faces and dt (p_{n+1} - p_{n-1}) / (x_{n+1} - x_{n-1}) of the cell velocity
 // in FP64 (reciprocal tables Gm.inv64), results stored in FP32; the
 // divergence of the projected faces in FP64 before they are rounded.
-// Software-pipelined along i: plane i + 1's operands are loaded before plane
-// i is computed.  Three blocks per SM (80 registers, a few bytes spilled):
-// the kernel is latency-bound, and the extra warps cut it from 452 to
-// 395 us per step on 512x256x128 against two blocks at 114 registers.
+// Blocks [0, T.count) march the interior's column segments with plane i + 1's
+// operands loaded before plane i is computed, the others take the faces below
+// the interior.  Bound by memory latency and FP64 issue: three blocks per SM.
+// 512x256x128: 353 us, against 401 us over the face box with four
+// divisions a cell.
 struct ProjectOps {
-    double pee, pn, ps, pt, pb;  // p at i + 2 (the ring's next), j +- 1, k +- 1
+    double pe, pn, ps, pt, pb;    // p at i + 1, j +- 1, k +- 1
     float ju[3], jus, jub, u[3];  // JU at the cell, JU1 at j - 1, JU2 at k - 1, U
 };
 
-__device__ __forceinline__ void load_project_ops(Vec3<const float> JU, Vec3<float> U,
-                                                 const double *p, long long c, long long sx,
-                                                 long long sy, bool cell, ProjectOps &o) {
-    o.pee = p[c + sx];
+__device__ __forceinline__ void load_project_ops(Vec3<const float> JU, Vec3<float> U, const double *p, int c,
+                                                 int sx, int sy, ProjectOps &o) {
+    o.pe = p[c + sx];
     o.pn = p[c + sy];
+    o.ps = p[c - sy];
     o.pt = p[c + 1];
+    o.pb = p[c - 1];
 #pragma unroll
     for (int m = 0; m < 3; m++) o.ju[m] = JU.c[m][c];
-    if (cell) {
-        o.ps = p[c - sy];
-        o.pb = p[c - 1];
-        o.jus = JU.c[1][c - sy];
-        o.jub = JU.c[2][c - 1];
+    o.jus = JU.c[1][c - sy];
+    o.jub = JU.c[2][c - 1];
 #pragma unroll
-        for (int m = 0; m < 3; m++) o.u[m] = U.c[m][c];
-    }
+    for (int m = 0; m < 3; m++) o.u[m] = U.c[m][c];
+}
+
+// a projected face: JU - dt A (dp / dx)
+__device__ __forceinline__ double proj_face32(float ju, double dt, double area, double dp, double inv) {
+    return (double)ju - dt * area * (dp * inv);
 }
 
 __global__ void __launch_bounds__(TILE_THREADS, 3)
 k_project32(StepParams P, Segments T, MixedGeom Gm, Vec3<float> U, Vec3<const float> JUin,
             Vec3<float> JUout, const double *p, Partials<2> part, DiagState *diag) {
     const Grid &g = P.g;
-    const long long sx = g.sx, sy = g.sy;
+    const int sx = (int)g.sx, sy = (int)g.sy;
     const double dt = P.dt;
     double div2 = 0, cfl = 0;
-    for (int u = blockIdx.x; u < T.count; u += gridDim.x) {
-        int i0, i1, j, k;
-        if (!T.column(u, i0, i1, j, k)) continue;
-        const bool jk_in = j >= g.gc && j < g.ny - g.gc && k >= g.gc && k < g.nz - g.gc;
-        const double uin = P.prof ? P.prof[((long long)j * g.nz + k) * 3] : P.uin[0];
-        const bool ywall_n = (j == g.gc - 1 || j == g.ny - g.gc - 1) && k >= g.gc && k < g.nz - g.gc;
-        const bool zwall_t = (k == g.gc - 1 || k == g.nz - g.gc - 1) && j >= g.gc && j < g.ny - g.gc;
-        const bool ywall_s = j - 1 == g.gc - 1 || j - 1 == g.ny - g.gc - 1;
-        const bool zwall_b = k - 1 == g.gc - 1 || k - 1 == g.nz - g.gc - 1;
-        long long c = g.at(i0, j, k);
-        double p_w = p[c - sx], p_c = p[c];
-        double fw = 0.0;
-        if (i0 > g.gc - 1)
-            fw = (i0 - 1 == g.gc - 1 && jk_in)
-                     ? P.m.dy[j] * P.m.dz[k] * uin
-                     : (double)JUin.c[0][c - sx] -
-                           dt * (P.m.dy[j] * P.m.dz[k]) * ((p_c - p_w) * Gm.inv64[0][i0 - 1].x);
-        ProjectOps cur{}, nxt{};
-        load_project_ops(JUin, U, p, c, sx, sy, jk_in && i0 >= g.gc, cur);
+    int i0, i1, j, k;
+    if ((int)blockIdx.x >= T.count) {
+        const long long step = (long long)(gridDim.x - T.count) * blockDim.x;
+        for (long long n = (long long)(blockIdx.x - T.count) * blockDim.x + threadIdx.x;
+             n < face_shell_cells(g); n += step) {
+            int i;
+            face_shell_cell(g, n, i, j, k);
+            const int c = (int)g.at(i, j, k);
+            const bool iin = i >= g.gc, jin = j >= g.gc, kin = k >= g.gc;  // (none is past the interior)
+            const bool wall_n = (j == g.gc - 1 || j == g.ny - g.gc - 1) && iin && kin;
+            const bool wall_t = (k == g.gc - 1 || k == g.nz - g.gc - 1) && iin && jin;
+            const double dx = P.m.dx[i], dy = P.m.dy[j], dz = P.m.dz[k], pc = p[c];
+            const double uin = P.prof ? P.prof[((long long)j * g.nz + k) * 3] : P.uin[0];
+            JUout.c[0][c] = (float)(!iin && jin && kin ? dy * dz * uin
+                                                       : proj_face32(JUin.c[0][c], dt, dy * dz, p[c + sx] - pc,
+                                                                     Gm.inv64[0][i].x));
+            JUout.c[1][c] = (float)(wall_n ? 0.0 : proj_face32(JUin.c[1][c], dt, dx * dz, p[c + sy] - pc,
+                                                               Gm.inv64[1][j].x));
+            JUout.c[2][c] = (float)(wall_t ? 0.0 : proj_face32(JUin.c[2][c], dt, dx * dy, p[c + 1] - pc,
+                                                               Gm.inv64[2][k].x));
+        }
+    } else if (T.column(blockIdx.x, i0, i1, j, k)) {
+        const bool wall_n = j == g.ny - g.gc - 1, wall_s = j == g.gc;
+        const bool wall_t = k == g.nz - g.gc - 1, wall_b = k == g.gc;
+        const double dy = P.m.dy[j], dz = P.m.dz[k], yz = dy * dz;
+        const double2 iy = Gm.inv64[1][j], iz = Gm.inv64[2][k];
+        const double iyS = Gm.inv64[1][j - 1].x, izB = Gm.inv64[2][k - 1].x;
+        const double idy = P.invd[1][j], idz = P.invd[2][k];
+        int c = (int)g.at(i0, j, k);
+        double pw = p[c - sx], pc = p[c];
+        double fw = i0 == g.gc
+                        ? dy * dz * (P.prof ? P.prof[((long long)j * g.nz + k) * 3] : P.uin[0])
+                        : proj_face32(JUin.c[0][c - sx], dt, yz, pc - pw, Gm.inv64[0][i0 - 1].x);
+        ProjectOps cur, nxt;
+        load_project_ops(JUin, U, p, c, sx, sy, cur);
         for (int i = i0; i < i1; i++, c += sx) {
-            const bool cell = jk_in && i >= g.gc && i < g.nx - g.gc;
-            if (i + 1 < i1)
-                load_project_ops(JUin, U, p, c + sx, sx, sy, jk_in && i + 1 >= g.gc && i + 1 < g.nx - g.gc,
-                                 nxt);
-            const double p_e = cur.pee;
-            const double dx = P.m.dx[i], dy = P.m.dy[j], dz = P.m.dz[k];
-            const bool iin = i >= g.gc && i < g.nx - g.gc;
-            const double fe = (i == g.gc - 1 && jk_in)
-                                  ? dy * dz * uin
-                                  : (double)cur.ju[0] - dt * (dy * dz) * ((p_e - p_c) * Gm.inv64[0][i].x);
-            const double fn = (ywall_n && iin)
-                                  ? 0.0
-                                  : (double)cur.ju[1] - dt * (dx * dz) * ((cur.pn - p_c) * Gm.inv64[1][j].x);
-            const double ft = (zwall_t && iin)
-                                  ? 0.0
-                                  : (double)cur.ju[2] - dt * (dx * dy) * ((cur.pt - p_c) * Gm.inv64[2][k].x);
+            if (i + 1 < i1) load_project_ops(JUin, U, p, c + sx, sx, sy, nxt);
+            const double dx = P.m.dx[i], xz = dx * dz, xy = dx * dy;
+            const double2 ix = Gm.inv64[0][i];
+            const double fe = proj_face32(cur.ju[0], dt, yz, cur.pe - pc, ix.x);
+            const double fn = wall_n ? 0.0 : proj_face32(cur.ju[1], dt, xz, cur.pn - pc, iy.x);
+            const double ft = wall_t ? 0.0 : proj_face32(cur.ju[2], dt, xy, cur.pt - pc, iz.x);
             JUout.c[0][c] = (float)fe;
             JUout.c[1][c] = (float)fn;
             JUout.c[2][c] = (float)ft;
-            if (cell) {
-                double uu = (double)cur.u[0] - dt * (p_e - p_w) * Gm.inv64[0][i].y;
-                double vv = (double)cur.u[1] - dt * (cur.pn - cur.ps) * Gm.inv64[1][j].y;
-                double ww = (double)cur.u[2] - dt * (cur.pt - cur.pb) * Gm.inv64[2][k].y;
-                if (P.solid) {  // set_solid_U (src/cfd.h:1143-1160)
-                    const double sf = P.solid[c];
-                    uu = (1. - sf) * uu;
-                    vv = (1. - sf) * vv;
-                    ww = (1. - sf) * ww;
-                }
-                U.c[0][c] = (float)uu;
-                U.c[1][c] = (float)vv;
-                U.c[2][c] = (float)ww;
-                const double fs = ywall_s ? 0.0
-                                          : (double)cur.jus -
-                                                dt * (dx * dz) * ((p_c - cur.ps) * Gm.inv64[1][j - 1].x);
-                const double fb = zwall_b ? 0.0
-                                          : (double)cur.jub -
-                                                dt * (dx * dy) * ((p_c - cur.pb) * Gm.inv64[2][k - 1].x);
-                const double d = (fe - fw + fn - fs + ft - fb) / (dx * dy * dz);
-                div2 += d * d;
-                const double local = (fabs(uu) / dx + fabs(vv) / dy + fabs(ww) / dz) * dt;
-                cfl = local > cfl ? local : cfl;
+            double uu = (double)cur.u[0] - dt * (cur.pe - pw) * ix.y;
+            double vv = (double)cur.u[1] - dt * (cur.pn - cur.ps) * iy.y;
+            double ww = (double)cur.u[2] - dt * (cur.pt - cur.pb) * iz.y;
+            if (P.solid) {  // set_solid_U (src/cfd.h:1143-1160)
+                const double sf = P.solid[c];
+                uu = (1. - sf) * uu;
+                vv = (1. - sf) * vv;
+                ww = (1. - sf) * ww;
             }
+            U.c[0][c] = (float)uu;
+            U.c[1][c] = (float)vv;
+            U.c[2][c] = (float)ww;
+            const double fs = wall_s ? 0.0 : proj_face32(cur.jus, dt, xz, pc - cur.ps, iyS);
+            const double fb = wall_b ? 0.0 : proj_face32(cur.jub, dt, xy, pc - cur.pb, izB);
+            const double d = (fe - fw + fn - fs + ft - fb) / (dx * dy * dz);
+            div2 += d * d;
+            const double local = (div_by(fabs(uu), dx, P.invd[0][i]) + div_by(fabs(vv), dy, idy) +
+                                  div_by(fabs(ww), dz, idz)) * dt;
+            cfl = local > cfl ? local : cfl;
             fw = fe;
-            p_w = p_c;
-            p_c = p_e;
+            pw = pc;
+            pc = cur.pe;
             cur = nxt;
         }
     }
@@ -509,10 +538,6 @@ k_project32(StepParams P, Segments T, MixedGeom Gm, Vec3<float> U, Vec3<const fl
 Box interior_box32(const Grid &g) {
     return Box{{g.gc, g.gc, g.gc}, {g.nx - g.gc, g.ny - g.gc, g.nz - g.gc}};
 }
-Box face_box32(const Grid &g) {
-    return Box{{g.gc - 1, g.gc - 1, g.gc - 1}, {g.nx - g.gc, g.ny - g.gc, g.nz - g.gc}};
-}
-
 }  // namespace
 
 void launch_predict32(const LaunchCtx &L, const StepParams &P, const MixedGeom &geo,
@@ -535,21 +560,23 @@ void launch_predict32(const LaunchCtx &L, const StepParams &P, const MixedGeom &
 
 void launch_flux32(const LaunchCtx &L, const StepParams &P, const MixedGeom &geo,
                    Vec3<const float> u, Vec3<float> ju, double *b) {
-    const Segments T = Segments::make(face_box32(P.g), L.blocks);
+    const Segments T = Segments::make(interior_box32(P.g), L.blocks);
+    const int blocks = T.count + shell_blocks(P.g, T);
     L.pre(KK_FLUX_RHS);
     if (b)
-        k_flux32<true><<<L.blocks, TILE_THREADS, 0, L.s>>>(P, T, geo, u, ju, b);
+        k_flux32<true><<<blocks, TILE_THREADS, 0, L.s>>>(P, T, geo, u, ju, b);
     else
-        k_flux32<false><<<L.blocks, TILE_THREADS, 0, L.s>>>(P, T, geo, u, ju, nullptr);
+        k_flux32<false><<<blocks, TILE_THREADS, 0, L.s>>>(P, T, geo, u, ju, nullptr);
     L.post(KK_FLUX_RHS);
 }
 
 void launch_project32(const LaunchCtx &L, const StepParams &P, const MixedGeom &geo, Vec3<float> u,
                       Vec3<const float> ju_in, Vec3<float> ju_out, const double *p,
                       Partials<2> part, DiagState *diag) {
-    const Segments T = Segments::make(face_box32(P.g), L.blocks);
+    const Segments T = Segments::make(interior_box32(P.g), L.blocks);
     L.pre(KK_PROJECT);
-    k_project32<<<L.blocks, TILE_THREADS, 0, L.s>>>(P, T, geo, u, ju_in, ju_out, p, part, diag);
+    k_project32<<<T.count + shell_blocks(P.g, T), TILE_THREADS, 0, L.s>>>(P, T, geo, u, ju_in, ju_out, p, part,
+                                                                        diag);
     L.post(KK_PROJECT);
 }
 
