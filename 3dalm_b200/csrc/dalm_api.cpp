@@ -51,8 +51,6 @@ constexpr double INNER_RTOL = 1e-4;
 constexpr long long INNER_CAP = 100;
 constexpr double STALL = 0.85;
 constexpr long long MAX_REFINE = 1000;
-// Largest grid whose coarse multigrid levels run as a cluster kernel.
-constexpr long long MG_CLUSTER_CELLS = 4000000;
 // Iterations per launch of a resident solve: bounds a launch to a fraction of a
 // second.
 constexpr long long RESIDENT_BUDGET = 1000;
@@ -519,11 +517,8 @@ struct dalm_handle {
             // mesh allows (on the coarser, latency-bound levels the table's
             // loads cost more than the elimination they save: measured on C4)
             MgLineTable &T = h.table;
-            // The cluster's warps read them once per visit, for several
-            // half-sweeps, and have them on every level.
-            const bool cluster = !opt.profile && geo[0].cells() <= MG_CLUSTER_CELLS;
-            h.has_table = (l < 2 || cluster) && mg_line_table(v.n, fcf, fw, T);
-            if (l < 2 && h.has_table) {
+            h.has_table = l < 2 && mg_line_table(v.n, fcf, fw, T);
+            if (h.has_table) {
                 v.lcls[0] = upload(T.cls[0]);
                 v.lcls[1] = upload(T.cls[1]);
                 v.lky = T.ky;
@@ -549,12 +544,11 @@ struct dalm_handle {
 
     // The levels that one cluster of blocks holds run as one kernel
     // (multigrid_cluster.cu), from the first level that fits (ms per step,
-    // launches / cluster: 64x32x40 1.31 / 0.90, 160x96x72 3.30 / 2.70).  On
-    // large grids those levels are a few percent of a step (512x256x128 4.39 /
-    // 4.34), and the launches stay.  Profiling times the half-sweeps' launches
-    // and keeps them.
+    // launches / cluster: 64x32x40 1.31 / 0.94, 160x96x72 3.30 / 2.80,
+    // 512x256x128 3.96 / 3.85), with the launches' bits.  Profiling times the
+    // half-sweeps' launches and keeps them.
     void setup_mg_cluster(const std::vector<MgLevelHost> &host) {
-        if (opt.profile || mgd.L[0].cells() > MG_CLUSTER_CELLS) return;
+        if (opt.profile) return;
         for (int first = 0; first + 1 < mgd.levels; first++) {
             MgCluster M;
             std::vector<float> image, tables;

@@ -72,16 +72,12 @@ struct MgRow {
         xw = L.cf[0][i];
         yn = L.cf[1][j + 1];
         ys = L.cf[1][j];
-        sxy = w1 * (xe + xw) + w0 * (yn + ys);
+        sxy = mg_line_sxy(w0, w1, xe, xw, yn, ys);
     }
     __device__ __forceinline__ float apply(const MgLevel &L, const float *x, int k) const {
         const float *xr = x + c0 + k;
-        const float w2 = L.w[2][k], zt = L.cf[2][k + 1], zb = L.cf[2][k];
-        const float diag = w2 * sxy + az * (zt + zb);
-        const float nb =
-            w2 * (w1 * (xe * xr[sx] + xw * xr[-sx]) + w0 * (yn * xr[sy] + ys * xr[-sy])) +
-            az * (zt * xr[1] + zb * xr[-1]);
-        return diag * xr[0] - nb;
+        return mg_cell_apply(L.w[2][k], w0, w1, az, sxy, xe, xw, yn, ys, L.cf[2][k + 1], L.cf[2][k], xr[0], xr[sx],
+                             xr[-sx], xr[sy], xr[-sy], xr[1], xr[-1]);
     }
 };
 
@@ -236,12 +232,12 @@ __global__ void __launch_bounds__(MG_THREADS, smooth_blocks(R)) k_mg_smooth_rows
 #pragma unroll
         for (int q = 0; q < R; q++)
             d[q] = zero ? v.f[q]
-                        : v.f[q] + w2[q] * (K.wj * (K.xe * v.e[q] + K.xw * v.w[q]) +
-                                            K.wi * (K.yn * v.n[q] + K.ys * v.s[q]));
+                        : mg_line_rhs(v.f[q], w2[q], K.wi, K.wj, K.xe, K.xw, K.yn, K.ys, v.e[q], v.w[q], v.n[q],
+                                      v.s[q]);
         if (FAC) {
             F.solve(lane, d, xs);
         } else {
-            const float az = K.wi * K.wj, sxy = K.wj * (K.xe + K.xw) + K.wi * (K.yn + K.ys);
+            const float az = K.wi * K.wj, sxy = mg_line_sxy(K.wi, K.wj, K.xe, K.xw, K.yn, K.ys);
             line_solve<R>(az, sxy, L.w[2], L.cf[2], L.n[2], lane, d, xs);
         }
         store_seg<R>(x + c, xs);
@@ -274,7 +270,7 @@ __device__ __forceinline__ void zline_solve_column(const ZlineArgs &A, int i, in
     // the column's constants (mg_zline_coef and mg_zline_rhs per row)
     const float wi = L.w[0][i], wj = L.w[1][j];
     const float xe = L.cf[0][i + 1], xw = L.cf[0][i], yn = L.cf[1][j + 1], ys = L.cf[1][j];
-    const float az = wi * wj, sxy = wj * (xe + xw) + wi * (yn + ys);
+    const float az = wi * wj, sxy = mg_line_sxy(wi, wj, xe, xw, yn, ys);
     const float *w2 = L.w[2], *cf2 = L.cf[2];
     // the column and its x and y neighbours, from k = 0
     const float *fr = f + c0, *xre = x + c0 + L.g.sx, *xrw = x + c0 - L.g.sx,
@@ -305,8 +301,7 @@ __device__ __forceinline__ void zline_solve_column(const ZlineArgs &A, int i, in
 #pragma unroll
         for (int q = 0; q < R; q++)
             d[q] = zero ? vf[q]
-                        : vf[q] + vw2[q] * (wj * (xe * ve[q] + xw * vw[q]) +
-                                            wi * (yn * vn[q] + ys * vs[q]));
+                        : mg_line_rhs(vf[q], vw2[q], wi, wj, xe, xw, yn, ys, ve[q], vw[q], vn[q], vs[q]);
     } else {
         // all of the column's loads first, then the slab
         float rhs[R];
@@ -325,7 +320,7 @@ __device__ __forceinline__ void zline_solve_column(const ZlineArgs &A, int i, in
                         if (pn >= 0) vn += xc[pn + K];
                         if (ps >= 0) vs += xc[ps + K];
                     }
-                    rhs[r] += w2[k] * (wj * (xe * ve + xw * vw) + wi * (yn * vn + ys * vs));
+                    rhs[r] = mg_line_rhs(rhs[r], w2[k], wi, wj, xe, xw, yn, ys, ve, vw, vn, vs);
                 }
             }
         }
@@ -608,15 +603,13 @@ __device__ __forceinline__ void row_apply(const MgLevel &L, const SpmvLoads<R> &
     const float up = __shfl_down_sync(full, v.c[0], 1);
     const float dn = __shfl_up_sync(full, v.c[R - 1], 1);
     const float az = w0 * w1;
-    const float sxy = w1 * (xe + xw) + w0 * (yn + ys);
+    const float sxy = mg_line_sxy(w0, w1, xe, xw, yn, ys);
 #pragma unroll
     for (int s = 0; s < R; s++) {
         const float bl = s > 0 ? v.c[s > 0 ? s - 1 : 0] : (lane == 0 ? v.below : dn);
         const float ab = s < R - 1 ? v.c[s < R - 1 ? s + 1 : 0] : (lane == 31 ? v.above : up);
-        const float diag = w2[s] * sxy + az * (zt[s] + zb[s]);
-        const float nb = w2[s] * (w1 * (xe * v.e[s] + xw * v.w[s]) + w0 * (yn * v.n[s] + ys * v.s[s])) +
-                         az * (zt[s] * ab + zb[s] * bl);
-        out[s] = diag * v.c[s] - nb;
+        out[s] = mg_cell_apply(w2[s], w0, w1, az, sxy, xe, xw, yn, ys, zt[s], zb[s], v.c[s], v.e[s], v.w[s], v.n[s],
+                               v.s[s], ab, bl);
     }
 }
 

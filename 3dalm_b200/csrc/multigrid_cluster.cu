@@ -15,17 +15,21 @@
 // most one column each per half-sweep, so levels with more columns than the
 // cluster has warps stay launches over the whole device (with four columns a
 // warp on the first level the kernel was slower than the launches it replaced).
-// So what a visit can do once is done once, before its half-sweeps: the line's
-// factors come from the tables, addresses and coefficients stay in registers,
-// and what lies past the grid is a column of zeros instead of a branch.
-// 64x32x40 took 0.98 ms a step with factors eliminated in each visit, generic
-// addresses and a spilled state, now 0.90; 160x96x72 2.89, now 2.70.  Small
-// levels whole in one block, with block barriers for cluster barriers, gained
-// nothing.
+// So what a visit can do once is done once, before its half-sweeps: the finer
+// levels' line factors come from their tables, addresses and coefficients stay
+// in registers, and what lies past the grid is a column of zeros instead of a
+// branch.  64x32x40 0.94 ms a step, 160x96x72 2.80 (0.98 and 2.89 with generic
+// addresses and a spilled state).  Factors formed once per visit or once per
+// handle on the other levels too took 0.90 and 2.70, but other roundings than
+// the launched kernels' elimination, and where the stop leaves the pressure
+// loose (128 cells along z at a small time step) those show as 1e-4 of it.
+// Small levels whole in one block, with block barriers for cluster barriers,
+// gained nothing.
 //
-// Operations are mg_vcycle's in the folded form of DeviceCycle (multigrid.cu):
-// the restriction leaves out the colour smoothed last, and a prolongation is
-// added to the neighbours by the half-sweep after it.
+// Operations are mg_vcycle's in the folded form of DeviceCycle (multigrid.cu),
+// and give the launched kernels' bits: the restriction leaves out the colour
+// smoothed last, and a prolongation is added to the neighbours by the
+// half-sweep after it.
 #include <algorithm>
 #include <type_traits>
 
@@ -144,20 +148,19 @@ struct Cycle {
             for (int s = 0; s < 2 * nu; s++) cluster_sync();
             return;
         }
-        LineFactors<R> F[2];
-        float f[2][R], w2[R], ke[2], kw[2], kn[2], ks[2];
+        LineFactors<R> F[2] = {};
+        float f[2][R], w2[R], wj[2], yn[2], ys[2];
         unsigned e[2], w[2];               // the neighbours' rows of this lane
         const float *nn[2], *ss[2];
         float *at[2];
         bool has[2];
         load_seg<R>(L.w2 + R * lane, w2);
+        const float wi = L.w0[i], xe = L.cf0[i + 1], xw = L.cf0[i];
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             const int jq = 2 * h + ((i + q) & 1), j = min(jq, n1 - 1), col = j * S + R * lane;
             has[q] = jq < n1;  // (an odd count's last: solved with the others, not stored)
-            const float wi = L.w0[i], xe = L.cf0[i + 1], xw = L.cf0[i];
-            const float wj = L.w1[j], yn = L.cf1[j + 1], ys = L.cf1[j];
-            ke[q] = wj * xe, kw[q] = wj * xw, kn[q] = wi * yn, ks[q] = wi * ys;
+            wj[q] = L.w1[j], yn[q] = L.cf1[j + 1], ys[q] = L.cf1[j];
             at[q] = L.x + ip * n1 * S + col;
             e[q] = i + 1 < n0 ? L.planes[i + 1] + 4 * col : zeros_at;
             w[q] = i > 0 ? L.planes[i - 1] + 4 * col : zeros_at;
@@ -166,8 +169,6 @@ struct Cycle {
             load_seg<R>(at[q] + (c.f - c.x), f[q]);
             if (c.tab >= 0)
                 F[q].load(tables + c.tab + (L.cls0[i] * c.lky + L.cls1[j]) * mglf_count(R) * 32 + lane);
-            else
-                F[q].factor(wi * wj, wj * (xe + xw) + wi * (yn + ys), L.w2, L.cf2, c.n[2], lane);
         }
         auto half = [&](auto colour, bool zero, bool pending) {
             constexpr int q = decltype(colour)::value;  // constant: the arrays stay in registers
@@ -197,9 +198,10 @@ struct Cycle {
                 }
 #pragma unroll
                 for (int t = 0; t < R; t++)
-                    d[t] += w2[t] * (ke[q] * ve[t] + kw[q] * vw[t] + (kn[q] * vn[t] + ks[q] * vs[t]));
+                    d[t] = mg_line_rhs(d[t], w2[t], wi, wj[q], xe, xw, yn[q], ys[q], ve[t], vw[t], vn[t], vs[t]);
             }
-            F[q].solve(lane, d, x);
+            if (c.tab >= 0) F[q].solve(lane, d, x);
+            else line_solve<R>(wi * wj[q], mg_line_sxy(wi, wj[q], xe, xw, yn[q], ys[q]), L.w2, L.cf2, c.n[2], lane, d, x);
             if (has[q]) store_seg<R>(at[q], x);
             cluster_sync();
         };
@@ -233,7 +235,7 @@ struct Cycle {
             s = j > 0 ? x - row : zeros_at;
             w0 = F.w0[i], w1 = F.w1[j], az = w0 * w1;
             ce = F.cf0[i + 1], cw = F.cf0[i], cn = F.cf1[j + 1], cs = F.cf1[j];
-            sxy = w1 * (ce + cw) + w0 * (cn + cs);
+            sxy = mg_line_sxy(w0, w1, ce, cw, cn, cs);
         }
         // f - K x at k
         __device__ __forceinline__ float residual(const Lv &F, int k) const {
@@ -242,9 +244,7 @@ struct Cycle {
             const float xe = load_word(e + o), xw = load_word(w + o), xn = load_word(n + o), xs = load_word(s + o);
             const float xt = k + 1 < F.c->n[2] ? load_word(x + o + 4) : 0.f, xb = k > 0 ? load_word(x + o - 4) : 0.f;
             const float w2 = F.w2[k], zt = F.cf2[k + 1], zb = F.cf2[k];
-            const float diag = w2 * sxy + az * (zt + zb);
-            const float nb = w2 * (w1 * (ce * xe + cw * xw) + w0 * (cn * xn + cs * xs)) + az * (zt * xt + zb * xb);
-            return rhs - (diag * xk - nb);
+            return rhs - mg_cell_apply(w2, w0, w1, az, sxy, ce, cw, cn, cs, zt, zb, xk, xe, xw, xn, xs, xt, xb);
         }
     };
 
@@ -265,14 +265,11 @@ struct Cycle {
             const Child B(F, i + fx - 1, odd || fy == 1 ? j : j + 1, zeros_at);
 #pragma unroll 1
             for (int K = lane; K < c.n[2]; K += 32) {
-                float sum = 0.f;
-#pragma unroll 1
-                for (int t = 0; t < c.fac[2]; t++) {
-                    const int k = K * c.fac[2] + t;
-                    const float ra = A.residual(F, k), rb = B.residual(F, k);
-                    sum += (one ? ra : 0.f) + (two ? rb : 0.f);
-                }
-                out[K] = sum;
+                const int k = K * c.fac[2];
+                const float a0 = A.residual(F, k), b0 = B.residual(F, k);
+                float a1 = 0.f, b1 = 0.f;
+                if (c.fac[2] == 2) a1 = A.residual(F, k + 1), b1 = B.residual(F, k + 1);
+                out[K] = (one ? a0 + a1 : 0.f) + (two ? b0 : 0.f) + (two ? b1 : 0.f);
             }
         }
         cluster_sync();

@@ -122,83 +122,40 @@ __device__ __forceinline__ void line_solve_table(const float *T, int lane, const
                                 T[32 * mglf_xc(s < R - 1 ? s : 0)] * y;
 }
 
-// The matrix-only part of a line solve, kept by a warp that solves the same
-// column several times: factor() and solve() together do line_solve's
-// operations, load() and solve() line_solve_table's.
+// a x + b y and the expressions of a cell built from it.  The fused products
+// are spelled out: the launched kernels and the cluster kernel then give the
+// same bits, whatever the compiler would fuse in either.
+__device__ __forceinline__ float mg_pair(float a, float x, float b, float y) {
+    return __fmaf_rn(a, x, __fmul_rn(b, y));
+}
+// a column's right-hand side at one cell: f + the x and y neighbours' terms
+__device__ __forceinline__ float mg_line_rhs(float f, float w2, float wi, float wj, float xe, float xw, float yn,
+                                             float ys, float e, float w, float n, float s) {
+    return __fmaf_rn(w2, mg_pair(wj, mg_pair(xe, e, xw, w), wi, mg_pair(yn, n, ys, s)), f);
+}
+// the x and y part of a column's diagonal, over w2
+__device__ __forceinline__ float mg_line_sxy(float wi, float wj, float xe, float xw, float yn, float ys) {
+    return mg_pair(wj, xe + xw, wi, yn + ys);
+}
+// (K x) at one cell, az = w0 w1
+__device__ __forceinline__ float mg_cell_apply(float w2, float w0, float w1, float az, float sxy, float xe, float xw,
+                                               float yn, float ys, float zt, float zb, float c, float e, float w,
+                                               float n, float s, float t, float b) {
+    const float diag = mg_pair(w2, sxy, az, zt + zb);
+    const float nb = mg_pair(w2, mg_pair(w1, mg_pair(xe, e, xw, w), w0, mg_pair(yn, n, ys, s)), az,
+                             mg_pair(zt, t, zb, b));
+    return __fmaf_rn(diag, c, -nb);
+}
+
+// A class's entry of the factor table in registers, for a warp that solves
+// several columns of the class, or one column several times: load() and
+// solve() do line_solve_table's operations.
 template <int R>
 struct LineFactors {
     static constexpr int H = R > 1 ? R - 1 : 1;
     float q[H], a[H], g[H], xa[H], xc[H];  // rows 0 .. R - 2
     float al, cl, alpha[5], gamma[5], last;
-    bool divide;  // last is the reduced diagonal (else its reciprocal)
 
-    __device__ __forceinline__ void factor(float az, float sxy, const float *w2, const float *cf2, int nk,
-                                           int lane) {
-        const unsigned full = 0xffffffffu;
-        float A[R], b[R], c[R];
-#pragma unroll
-        for (int s = 0; s < R; s++) {
-            const int k = R * lane + s;
-            if (k < nk) {
-                const float lo = az * cf2[k], hi = az * cf2[k + 1];
-                A[s] = -lo;
-                b[s] = w2[k] * sxy + lo + hi;
-                c[s] = -hi;
-            } else {
-                A[s] = 0.f;
-                b[s] = 1.f;
-                c[s] = 0.f;
-            }
-        }
-        float ra = A[R - 1], rb = b[R - 1], rc = c[R - 1];
-        if (R > 1) {
-            float fa[R], gg[R];
-#pragma unroll
-            for (int s = 0; s < R - 1; s++) {
-                const float den = s == 0 ? b[0] : b[s] - A[s] * gg[s > 0 ? s - 1 : 0];
-                const float qq = __fdividef(1.f, den);
-                fa[s] = (s == 0 ? A[0] : -A[s] * fa[s > 0 ? s - 1 : 0]) * qq;
-                gg[s] = c[s] * qq;
-                q[s] = qq;
-                a[s] = A[s];
-                g[s] = gg[s];
-            }
-#pragma unroll
-            for (int s = R - 3; s >= 0; s--) {
-                fa[s] -= gg[s] * fa[s + 1];
-                gg[s] = -gg[s] * gg[s + 1];
-            }
-            float An = __shfl_down_sync(full, fa[0], 1), Cn = __shfl_down_sync(full, gg[0], 1);
-            if (lane == 31) An = Cn = 0.f;
-            al = A[R - 1];
-            cl = lane == 31 ? 0.f : c[R - 1];
-            ra = -al * fa[R - 2];
-            rb = b[R - 1] - al * gg[R - 2] - c[R - 1] * An;
-            rc = -c[R - 1] * Cn;
-#pragma unroll
-            for (int s = 0; s < R - 1; s++) {
-                xa[s] = fa[s];
-                xc[s] = gg[s];
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 5; t++) {
-            const int delta = 1 << t;
-            float am = __shfl_up_sync(full, ra, delta), bm = __shfl_up_sync(full, rb, delta);
-            float cm = __shfl_up_sync(full, rc, delta);
-            float ap = __shfl_down_sync(full, ra, delta), bp = __shfl_down_sync(full, rb, delta);
-            float cp = __shfl_down_sync(full, rc, delta);
-            if (lane < delta) am = 0.f, bm = 1.f, cm = 0.f;
-            if (lane + delta >= 32) ap = 0.f, bp = 1.f, cp = 0.f;
-            alpha[t] = -__fdividef(ra, bm);
-            gamma[t] = -__fdividef(rc, bp);
-            rb += alpha[t] * cm + gamma[t] * ap;
-            ra = alpha[t] * am;
-            rc = gamma[t] * cp;
-        }
-        last = rb;
-        divide = true;
-    }
     __device__ __forceinline__ void load(const float *T) {
 #pragma unroll
         for (int s = 0; s < R - 1; s++) {
@@ -218,7 +175,6 @@ struct LineFactors {
             gamma[t] = T[32 * mglf_gamma(R, t)];
         }
         last = T[32 * mglf_invrb(R)];
-        divide = false;
     }
     __device__ __forceinline__ void solve(int lane, const float (&d)[R], float (&x)[R]) const {
         const unsigned full = 0xffffffffu;
@@ -241,7 +197,7 @@ struct LineFactors {
             if (lane + delta >= 32) dp = 0.f;
             rd += alpha[t] * dm + gamma[t] * dp;
         }
-        const float y = divide ? __fdividef(rd, last) : rd * last;
+        const float y = rd * last;
         float ym = __shfl_up_sync(full, y, 1);
         if (lane == 0) ym = 0.f;
 #pragma unroll
