@@ -9,6 +9,9 @@ namespace dalm {
 
 namespace {
 
+// dynamic shared memory of either kernel at most
+constexpr size_t ALM_SMEM = 200 * 1024;
+
 __device__ __forceinline__ double sq(double v) { return v * v; }
 
 // update_ap_position + calc_ap_force (src/alm.h:233-370) and the turbine's
@@ -189,9 +192,9 @@ void launch_alm_points(const LaunchCtx &L, const StepParams &P, const AlmDev &A,
     if (A.ap_count <= 0) return;
     // the sums' terms, the mesh and the polar angles in shared memory
     const size_t bytes = sizeof(double) * (2 * (size_t)A.ap_per_wt + P.g.nx + P.g.ny + P.g.nz + A.atk_count);
-    const bool staged = bytes <= 200 * 1024;
+    const bool staged = bytes <= ALM_SMEM;
     const size_t smem = staged ? bytes : 0;
-    DALM_CUDA(cudaFuncSetAttribute(k_alm_points<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(k_alm_points<T>, ALM_SMEM);
     const int threads = std::min(512, std::max(128, (A.ap_per_wt + 31) / 32 * 32));
     L.pre(KK_ALM_POINTS);
     k_alm_points<T><<<A.wt_count, threads, smem, L.s>>>(P, A, t, u, staged);
@@ -210,7 +213,7 @@ void launch_alm_project(const LaunchCtx &L, const StepParams &P, const AlmDev &A
     const int nti = (box.hi[0] - box.lo[0] + PP - 1) / PP;
     const size_t smem = sizeof(int) * (size_t)A.ap_count;
     if (smem > 32 * 1024)
-        DALM_CUDA(cudaFuncSetAttribute(k_alm_project<FT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared(k_alm_project<FT>, ALM_SMEM);
     L.pre(KK_ALM_PROJECT);
     k_alm_project<FT><<<ntk * ntj * nti, TILE_THREADS, smem, L.s>>>(P, A, box, ntk, ntj, f);
     L.post(KK_ALM_PROJECT);

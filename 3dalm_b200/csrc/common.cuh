@@ -309,6 +309,16 @@ inline void pdl_launch(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t sme
     DALM_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...));
 }
 
+// Allows launches of `kernel` with up to `bytes` of dynamic shared memory.
+// The limit belongs to the function in the device's context, not to a handle,
+// and a launch above it fails: `bytes` is the most the kernel ever takes, the
+// same value on every call, so that no handle lowers the limit between another
+// one's call and launch.
+template <typename K>
+inline void allow_shared(K kernel, size_t bytes) {
+    DALM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 inline int reduction_blocks(int sm_count) { return sm_count * 8; }
 
 }  // namespace dalm

@@ -554,7 +554,7 @@ struct dalm_handle {
             std::vector<float> image, tables;
             for (int blocks : {16, 8}) {  // 16: beyond the portable size, where the device takes it
                 M.top = mgd.L[first];
-                if (!mg_cluster_layout(host, first, blocks, MG_CLUSTER_WARPS, 220 * 1024, M, image, tables) || !mg_cluster_fits(M)) continue;
+                if (!mg_cluster_layout(host, first, blocks, MG_CLUSTER_WARPS, MG_CLUSTER_SMEM, M, image, tables) || !mg_cluster_fits(M)) continue;
                 M.kinv = mgd.kinv;
                 M.image = upload(image);
                 M.tables = tables.empty() ? nullptr : upload(tables);

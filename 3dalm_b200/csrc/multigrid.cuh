@@ -259,7 +259,8 @@ struct MgClusterLevel {
     int gather;                     // coarsest level: room for the whole f
     int planes;                     // [n[0]] addresses of the planes of x, wherever they are
 };
-constexpr int MG_CLUSTER_WARPS = 16;  // per block
+constexpr int MG_CLUSTER_WARPS = 16;              // per block
+constexpr size_t MG_CLUSTER_SMEM = 220 * 1024;    // dynamic shared memory per block at most
 // The levels from `first` on, for one cluster of `blocks` blocks.
 struct MgCluster {
     int first = 0, levels = 0;  // levels 0: not used

@@ -382,7 +382,7 @@ cudaLaunchConfig_t config(const MgCluster &M, cudaLaunchAttribute *attr, cudaStr
 auto kernel_of(const MgCluster &M) {
     const int R = (M.top.n[2] + 31) / 32;
     auto k = R == 1 ? k_mg_cluster<1> : R == 2 ? k_mg_cluster<2> : R == 3 ? k_mg_cluster<3> : k_mg_cluster<4>;
-    DALM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, M.total * 4));
+    allow_shared(k, MG_CLUSTER_SMEM);
     DALM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     return k;
 }

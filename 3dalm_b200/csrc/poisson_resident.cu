@@ -862,10 +862,15 @@ k_resident_bicg_sor(Grid g, PoissonCoef C, Cells cells, PoissonBufs B, int sweep
     finish(S, st, !ok);
 }
 
+// Dynamic shared memory of the kernels at most: the axis tables of
+// resident_available, the packed colours of one block, or three coefficients
+// per plane.
+constexpr size_t AXIS_SMEM = 200 * 1024, PACKED_SMEM = 150 * 1024, RESIDENT_SMEM = 208 * 1024;
+
 template <typename K, typename... Args>
 void cooperative(const LaunchCtx &L, K kernel, int blocks, int threads, size_t smem, Args... args) {
     void *ptrs[] = {(void *)&args...};
-    DALM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(kernel, RESIDENT_SMEM);
     L.pre(KK_RESIDENT);
     DALM_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(blocks), dim3(threads), ptrs, smem, L.s));
     L.post(KK_RESIDENT);
@@ -894,7 +899,7 @@ bool resident_available(const PoissonConfig &cfg, const Grid &g) {
         return false;
     // Divisor's range, and the axis tables' shared memory
     return g.nj() >= 2 && g.nk() >= 3 && cells * (unsigned long long)(g.nj() + g.nk()) < (1ull << 32) &&
-           AxisCoef::bytes(g) <= 200 * 1024;
+           AxisCoef::bytes(g) <= AXIS_SMEM;
 }
 
 void launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
@@ -919,7 +924,7 @@ void launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef 
     if (cfg.method == PM_SOR) {
         const Packed Q = Packed::make(cfg.seg.box);
         const size_t axis = 3 * sizeof(double) * (size_t)(Q.ni + SOR_UI), packed = 2 * sizeof(double) * (size_t)Q.total();
-        if (Q.threads <= RT && packed <= 150 * 1024) {
+        if (Q.threads <= RT && packed <= PACKED_SMEM) {
             cooperative(L, k_resident_sor_regs<true>, 1, RT, axis + packed, g, C, cfg.seg.box, Q, B.x, B.tp, B.ts, B.b,
                         cfg.relax, budget, part, sync, st);
             return;
