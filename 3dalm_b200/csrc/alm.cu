@@ -211,9 +211,10 @@ void launch_alm_project(const LaunchCtx &L, const StepParams &P, const AlmDev &A
     if (A.ap_count <= 0 || box.empty()) return;
     const int ntk = (box.hi[2] - box.lo[2] + TK - 1) / TK, ntj = (box.hi[1] - box.lo[1] + TJ - 1) / TJ;
     const int nti = (box.hi[0] - box.lo[0] + PP - 1) / PP;
+    // the list of points, beside 22 KB of static tables: with more than 6712
+    // points over the 48 KB that need no leave
     const size_t smem = sizeof(int) * (size_t)A.ap_count;
-    if (smem > 32 * 1024)
-        allow_shared(k_alm_project<FT>, ALM_SMEM);
+    allow_shared(k_alm_project<FT>, ALM_SMEM);
     L.pre(KK_ALM_PROJECT);
     k_alm_project<FT><<<ntk * ntj * nti, TILE_THREADS, smem, L.s>>>(P, A, box, ntk, ntj, f);
     L.post(KK_ALM_PROJECT);
