@@ -26,6 +26,7 @@
 #include "multigrid_setup.hpp"
 #include "output_io.hpp"
 #include "poisson.cuh"
+#include "scratch.hpp"
 
 using namespace dalm;
 
@@ -1534,33 +1535,17 @@ struct dalm_handle {
     } adj_stats;
     long long adj_hint = 0;
 
-    // Device buffers of one gradient run, cut from chunks of `chunk` bytes and
-    // freed when it ends (an allocation per buffer, some ninety of them, took
-    // a quarter of a small run's time).
-    struct Scratch {
-        size_t chunk, left = 0;
-        char *next = nullptr;
-        std::vector<void *> ptrs;
-        explicit Scratch(size_t bytes) : chunk(bytes) {}
-        ~Scratch() {
-            for (void *p : ptrs) cudaFree(p);
+    // device buffers of one gradient run, freed when it ends (an allocation per
+    // buffer, some ninety of them, took a quarter of a small run's time)
+    struct DeviceMem {
+        static void *allocate(size_t bytes) {
+            void *p = nullptr;
+            DALM_CUDA(cudaMalloc(&p, bytes));
+            return p;
         }
-        template <typename T>
-        T *get(size_t n) {
-            const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
-            if (bytes > left) {
-                void *p = nullptr;
-                left = std::max(chunk, bytes);
-                DALM_CUDA(cudaMalloc(&p, left));
-                ptrs.push_back(p);
-                next = (char *)p;
-            }
-            T *r = (T *)next;
-            next += bytes;
-            left -= bytes;
-            return r;
-        }
+        static void release(void *p) { cudaFree(p); }
     };
+    using Scratch = dalm::Scratch<DeviceMem>;
     // a restart point: the fields a step reads and the host-side step state
     struct Snapshot {
         double *U[3], *JU[3], *F[3], *p;
@@ -1744,9 +1729,9 @@ struct dalm_handle {
         alm_at(t_init);
 
         const int64_t nsteps = t1 - n_first + 1, nseg = (nsteps + k - 1) / k;
-        // restart points, tape and adjoint fields, in chunks of up to 256 MB
+        // restart points, tape and adjoint fields
         const size_t fields = 10 * ((size_t)nseg + 1) + 6 * (size_t)k + 6 + 20;
-        Scratch S(std::min<size_t>(fields * sizeof(double) * (size_t)g.total + (1 << 20), 256u << 20));
+        Scratch S(fields, sizeof(double) * (size_t)g.total);
         const int64_t last0 = n_first + (nseg - 1) * k;  // first step of the last segment
         std::vector<Snapshot> ck((size_t)nseg);
         for (auto &c : ck) alloc_snapshot(S, c);
