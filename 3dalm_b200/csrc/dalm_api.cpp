@@ -55,6 +55,9 @@ constexpr long long MAX_REFINE = 1000;
 // Iterations per launch of a resident solve: bounds a launch to a fraction of a
 // second.
 constexpr long long RESIDENT_BUDGET = 1000;
+// Polls of one barrier wait of a resident solve, about a second; less by the
+// environment's DALM_BARRIER_POLLS.
+constexpr unsigned WAIT_POLLS = 1u << 21;
 // Adjoint pressure solves stop at this RMS residual relative to the RMS of
 // their right-hand side.
 constexpr double ADJ_RTOL = 1e-10;
@@ -373,6 +376,9 @@ struct dalm_handle {
         pcfg.reference_sums = opt.reference_sums ? 1 : 0;
         pcfg.jacobi2 = opt.fused_jacobi ? 1 : 0;
         pcfg.sm_count = sm_count;
+        pcfg.wait_polls = WAIT_POLLS;
+        if (const char *polls = std::getenv("DALM_BARRIER_POLLS"))
+            pcfg.wait_polls = (unsigned)std::min<long long>(WAIT_POLLS, std::max<long long>(1, std::atoll(polls)));
         pcfg.seg = poisson_segments(g, sm_count);
         choose_route();
         // FP32 inner solves exist for BiCGStab only; SOR and Jacobi solves

@@ -67,6 +67,7 @@ struct PoissonConfig {
     int reference_sums;  // 1: global sums in the reference's serial order
     int jacobi2;         // 1: FP64 Jacobi(3): the last two sweeps in one pass
     int sm_count;
+    unsigned wait_polls; // limit of a resident solve's barrier wait
     Segments seg;        // column segments of the interior (one per block)
     const MapTable *maps;
 };

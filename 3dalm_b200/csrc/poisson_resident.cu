@@ -29,9 +29,11 @@
 // order (poisson_math.cuh), or on the off-diagonal part where the cells are in
 // registers; sums differ in their order.
 //
-// A barrier that does not complete within BARRIER_POLLS polls marks the solve
-// failed; every block then leaves at its next barrier, and the host reports
-// DALM_ERR_DEVICE_WAIT.
+// A block whose barrier does not complete within its polls marks the solve's
+// state and leaves; the others leave at their next barrier.  A straggler may
+// still find a barrier complete that another block gave up, so the mark is
+// never written over (finish), and the host reports DALM_ERR_DEVICE_WAIT
+// whatever else the state says.
 #include "poisson.cuh"
 #include "poisson_math.cuh"
 
@@ -39,8 +41,7 @@ namespace dalm {
 
 namespace {
 
-constexpr int RT = 512;                       // threads of the sweep kernels
-constexpr unsigned BARRIER_POLLS = 1u << 21;  // about a second
+constexpr int RT = 512;  // threads of the sweep kernels
 
 // The grid's barrier and sums.  One thread of a block adds 1 to a counter
 // (release) and polls it (acquire) until every block has: 2441 cycles over 148
@@ -52,9 +53,10 @@ constexpr unsigned BARRIER_POLLS = 1u << 21;  // about a second
 struct GridSync {
     unsigned *count;  // [0] arrivals, [1] failed; zeroed before the launch
     double2 *part;    // [2][gridDim.x]
+    unsigned polls;   // of one wait at most
     unsigned goal = 0;
     int set = 0;
-    __device__ GridSync(unsigned *c, double *p) : count(c), part((double2 *)p) {}
+    __device__ GridSync(unsigned *c, double *p, unsigned limit) : count(c), part((double2 *)p), polls(limit) {}
     static __device__ __forceinline__ unsigned load(const unsigned *p) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -65,7 +67,7 @@ struct GridSync {
         goal += gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         for (unsigned n = 0; (int)(load(count) - goal) < 0;) {
-            if (++n >= BARRIER_POLLS || ((n & 255u) == 0 && load(count + 1))) {
+            if (++n >= polls || ((n & 255u) == 0 && load(count + 1))) {
                 atomicExch(count + 1, 1u);
                 return false;
             }
@@ -250,9 +252,12 @@ __device__ __forceinline__ void for_cells(const Domain &D, int color, F body) {
 
 __device__ __forceinline__ void finish(const KrylovState &S, KrylovState *st, bool failed) {
     __syncthreads();
-    if (threadIdx.x == 0 && (blockIdx.x == 0 || failed)) {
-        if (!failed) *st = S;
-        else st->wait_error = 1, st->done = 1;
+    if (threadIdx.x != 0) return;
+    if (failed) {
+        st->wait_error = 1;
+    } else if (blockIdx.x == 0) {  // what a solve changes, but for the mark
+        st->rho = S.rho, st->rho_old = S.rho_old, st->alpha = S.alpha, st->omega = S.omega, st->beta = S.beta;
+        st->err = S.err, st->it = S.it, st->done = S.done, st->breakdown = S.breakdown;
     }
 }
 
@@ -262,7 +267,7 @@ __device__ __forceinline__ void finish(const KrylovState &S, KrylovState *st, bo
 // red cells of the other time level.
 __global__ void __launch_bounds__(RT, 1)
 k_resident_sor(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, const double *b, double w,
-               long long budget, double *part, unsigned *sync, KrylovState *st) {
+               long long budget, double *part, unsigned *sync, unsigned polls, KrylovState *st) {
     constexpr int U = 4;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
@@ -271,7 +276,7 @@ k_resident_sor(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, const
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part);
+    GridSync grid(sync, part, polls);
     double *cur = x, *nxt = tmp;  // red cells
     double black = 0.0;           // this thread's squared residuals at the black cells
     bool ok = true;
@@ -363,14 +368,14 @@ template <bool ONE>  // ONE: a single block, the packed arrays in its shared mem
 __global__ void __launch_bounds__(RT, 1)
 k_resident_sor_regs(Grid g, PoissonCoef C, Box box, Packed Q, double *x, double *red, double *blk,
                     const double *b, double w, long long budget, double *part, unsigned *sync,
-                    KrylovState *st) {
+                    unsigned polls, KrylovState *st) {
     constexpr int U = SOR_UI;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part);
+    GridSync grid(sync, part, polls);
     if (ONE) {
         red = resident_smem + 3 * (Q.ni + U);
         blk = red + Q.total();
@@ -501,7 +506,7 @@ k_resident_sor_regs(Grid g, PoissonCoef C, Box box, Packed Q, double *x, double 
 // Up to `budget` Jacobi iterations from x; tmp holds the other iterate.
 __global__ void __launch_bounds__(RT, 1)
 k_resident_jacobi(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, const double *b,
-                  long long budget, double *part, unsigned *sync, KrylovState *st) {
+                  long long budget, double *part, unsigned *sync, unsigned polls, KrylovState *st) {
     constexpr int U = 4;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
@@ -510,7 +515,7 @@ k_resident_jacobi(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, co
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part);
+    GridSync grid(sync, part, polls);
     double *cur = x, *nxt = tmp;
     bool ok = true;
     for (long long n = 0;; n++) {
@@ -604,13 +609,13 @@ struct Columns {
 template <int U, bool MEM>
 __global__ void __launch_bounds__(RT, 1)
 k_resident_bicg(Grid g, PoissonCoef C, Columns Q, PoissonBufs B, long long budget, double *part,
-                unsigned *sync, KrylovState *st) {
+                unsigned *sync, unsigned polls, KrylovState *st) {
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part);
+    GridSync grid(sync, part, polls);
     const Box &bx = Q.box;
     const int ni = bx.hi[0] - bx.lo[0];
     double *ci = resident_smem;  // coefficients along i, 0 past the interior
@@ -791,7 +796,7 @@ __device__ __forceinline__ void relax_color(const Domain &D, double *z, const do
 // update of v.
 __global__ void __launch_bounds__(RT, 1)
 k_resident_bicg_sor(Grid g, PoissonCoef C, Cells cells, PoissonBufs B, int sweeps, double w,
-                    long long budget, double *part, unsigned *sync, KrylovState *st) {
+                    long long budget, double *part, unsigned *sync, unsigned polls, KrylovState *st) {
     constexpr int U = 4;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
@@ -800,7 +805,7 @@ k_resident_bicg_sor(Grid g, PoissonCoef C, Cells cells, PoissonBufs B, int sweep
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part);
+    GridSync grid(sync, part, polls);
     bool ok = true;
     // v = update(c), z = M^-1 v, av = A z; v's sums with f: <f, av> or <av, v>, <av, av>
     auto half = [&](auto update, double *vv, double *z, double *av, const double *f, auto fin) {
@@ -883,7 +888,7 @@ bool resident_bicg(const LaunchCtx &L, const Grid &g, const PoissonCoef &C, cons
     const Columns Q = Columns::make(cfg.seg.box, U);
     if (Q.threads > (unsigned)cfg.sm_count * RT) return false;
     cooperative(L, k_resident_bicg<U, MEM>, (int)((Q.threads + RT - 1) / RT), RT,
-                3 * sizeof(double) * (size_t)(g.ni() + U), g, C, Q, B, budget, part, sync, st);
+                3 * sizeof(double) * (size_t)(g.ni() + U), g, C, Q, B, budget, part, sync, cfg.wait_polls, st);
     return true;
 }
 
@@ -926,22 +931,22 @@ void launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef 
         const size_t axis = 3 * sizeof(double) * (size_t)(Q.ni + SOR_UI), packed = 2 * sizeof(double) * (size_t)Q.total();
         if (Q.threads <= RT && packed <= PACKED_SMEM) {
             cooperative(L, k_resident_sor_regs<true>, 1, RT, axis + packed, g, C, cfg.seg.box, Q, B.x, B.tp, B.ts, B.b,
-                        cfg.relax, budget, part, sync, st);
+                        cfg.relax, budget, part, sync, cfg.wait_polls, st);
             return;
         }
         if (Q.threads <= (unsigned)cfg.sm_count * RT) {
             cooperative(L, k_resident_sor_regs<false>, (int)((Q.threads + RT - 1) / RT), RT, axis, g, C, cfg.seg.box,
-                        Q, B.x, B.tp, B.ts, B.b, cfg.relax, budget, part, sync, st);
+                        Q, B.x, B.tp, B.ts, B.b, cfg.relax, budget, part, sync, cfg.wait_polls, st);
             return;
         }
         cooperative(L, k_resident_sor, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, cfg.relax, budget,
-                    part, sync, st);
+                    part, sync, cfg.wait_polls, st);
     } else if (cfg.method == PM_JACOBI)
         cooperative(L, k_resident_jacobi, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, budget, part,
-                    sync, st);
+                    sync, cfg.wait_polls, st);
     else
         cooperative(L, k_resident_bicg_sor, blocks, RT, smem, g, C, cells, B, cfg.pc_sweeps, cfg.pc_relax,
-                    budget, part, sync, st);
+                    budget, part, sync, cfg.wait_polls, st);
 }
 
 }  // namespace dalm

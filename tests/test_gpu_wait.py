@@ -1,0 +1,36 @@
+"""A barrier wait of a resident solve that runs out (DALM_BARRIER_POLLS=1: one
+poll, before the other blocks can have arrived) is reported, by every step, and
+other handles are not touched by it."""
+import pytest
+
+from conftest import package
+
+pytestmark = pytest.mark.gpu
+
+
+# one launch's worth of iterations (the step does not wait for the solve), and
+# more (it does)
+@pytest.mark.parametrize("name,n", [("tiny-sor", (64, 40, 40)), ("tiny-sor", (97, 80, 79)),
+                                    ("tiny-jacobi", (64, 40, 40)), ("tiny-bicg", (63, 41, 40)),
+                                    ("tiny-sorpc", (64, 40, 40))])
+@pytest.mark.parametrize("its", [100, 3000])
+def test_wait_runs_out(make_case, monkeypatch, name, n, its):
+    pkg = package()
+    spec, mesh, d, U0, prof = make_case(name, n=n, dt=1e-4)
+    monkeypatch.setenv("DALM_BARRIER_POLLS", "1")
+    s = pkg.Solver(d)
+    monkeypatch.delenv("DALM_BARRIER_POLLS")
+    good = pkg.Solver(d)
+    for h in (s, good):
+        h.set_state(U0)
+        h.set_poisson(its, 0.0)
+        h.step(1)  # step 0: no solve
+    for _ in range(20):
+        with pytest.raises(pkg.DalmError) as e:
+            s.step(1)
+        assert e.value.code == 5, e.value
+        s.stats()  # reported once
+    good.step(2)
+    assert good.stats()["it"] > 0
+    s.finalize()
+    good.finalize()
