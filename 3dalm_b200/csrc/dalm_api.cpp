@@ -787,8 +787,8 @@ struct dalm_handle {
         states_ahead = false;
         check_waits();
     }
-    // A bounded device wait that ran out stays marked in the state over later
-    // solves until it is reported here.
+    // A bounded device wait that ran out stays marked in the state, and later
+    // solves return at once, until it is reported here.
     void check_waits() {
         if (!h_kst[0].wait_error && !h_kst[1].wait_error) return;
         for (int q = 0; q < 2; q++) {
@@ -1360,6 +1360,9 @@ struct dalm_handle {
     // file (time-averaged U) once averaging has started, and snapshot.json.
     void write_outputs() {
         const double t = cs.dt * (double)step;
+        const bool due = t - 0.5 * cs.dt < next_output_time && next_output_time <= t + 0.5 * cs.dt;
+        // nothing is written of a step whose solve's wait ran out
+        if (states_ahead && (due || !probe_list.empty())) sync_stats();
         record_probes(t);
         if (turbine_log.is_open() && step != 0) {
             sync_stats();
@@ -1375,7 +1378,7 @@ struct dalm_handle {
             turbine_log << "\n";
             turbine_log.flush();
         }
-        if (!(t - 0.5 * cs.dt < next_output_time && next_output_time <= t + 0.5 * cs.dt)) return;
+        if (!due) return;
         next_output_time += cs.output_interval_time;
         widen_state();
         const size_t cells = (size_t)g.nx * g.ny * g.nz;
@@ -1766,8 +1769,7 @@ struct dalm_handle {
             if (n >= last0) record(n - last0, true);
             step_once();
             if (n >= t0) {
-                fetch_step_outputs();
-                DALM_CUDA(cudaStreamSynchronize(stream));
+                sync_stats();
                 for (int w = 0; w < T; w++) J += h_wt_out[w] * std::fabs(h_wt[w].rot_speed);
             }
         }
@@ -1780,8 +1782,7 @@ struct dalm_handle {
         KrylovState *fin_kst = S.get<KrylovState>(2);
         DALM_CUDA(cudaMemcpyAsync(fin_diag, d_diag, sizeof(DiagState), cudaMemcpyDeviceToDevice, stream));
         DALM_CUDA(cudaMemcpyAsync(fin_kst, d_kst, 2 * sizeof(KrylovState), cudaMemcpyDeviceToDevice, stream));
-        fetch_step_outputs();
-        DALM_CUDA(cudaStreamSynchronize(stream));
+        sync_stats();
         KrylovState fin_hkst[2] = {h_kst[0], h_kst[1]};
         DiagState fin_hdiag = *h_diag;
         std::vector<double> fin_wt(h_wt_out, h_wt_out + 2 * T);
@@ -1839,6 +1840,7 @@ struct dalm_handle {
         std::vector<double> g_dev(3 * (size_t)T);
         DALM_CUDA(cudaMemcpyAsync(g_dev.data(), A.grad, sizeof(double) * 3 * T, cudaMemcpyDeviceToHost, stream));
         DALM_CUDA(cudaStreamSynchronize(stream));
+        states_ahead = false;
         h_kst[0] = fin_hkst[0];
         h_kst[1] = fin_hkst[1];
         *h_diag = fin_hdiag;

@@ -74,8 +74,11 @@ int kk(int k) {
 __global__ void k_begin(KrylovState *st, long long max_it, double tol, double ncell,
                         long long max_outer, double inner_rtol, long long inner_cap, int guard) {
     st->rho = 0; st->rho_old = 1; st->alpha = 1; st->omega = 1; st->beta = 0; st->err = 0;
-    st->ncell = ncell; st->tol = tol; st->it = 0; st->max_it = max_it; st->done = 0;
-    st->outer_it = 0;  // (wait_error stays until the host has seen it)
+    st->ncell = ncell; st->tol = tol; st->it = 0; st->max_it = max_it;
+    // a wait that ran out stays marked until the host has seen it, and no
+    // further solve runs on what it left
+    st->done = st->wait_error ? 1 : 0;
+    st->outer_it = 0;
     st->max_outer = max_outer; st->inner_rtol = inner_rtol;
     st->inner_cap = inner_cap; st->guard = guard; st->breakdown = 0;
 }

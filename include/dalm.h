@@ -35,7 +35,10 @@ extern "C" {
 #define DALM_ERR_CASE 2         /* unreadable / inconsistent case JSON        */
 #define DALM_ERR_CUDA 3         /* CUDA runtime error or no usable GPU        */
 #define DALM_ERR_NONFINITE 4    /* NaN/Inf detected in the state              */
-#define DALM_ERR_DEVICE_WAIT 5  /* a capped device-side wait ran out          */
+#define DALM_ERR_DEVICE_WAIT 5  /* a capped device-side wait ran out; the
+                                   call's later steps may have been taken
+                                   on the unfinished pressure: set the state
+                                   anew                                    */
 #define DALM_ERR_UNSUPPORTED 6  /* option combination not implemented         */
 
 /* ---- enums ------------------------------------------------------------ */

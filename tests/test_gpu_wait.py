@@ -34,3 +34,24 @@ def test_wait_runs_out(make_case, monkeypatch, name, n, its):
     assert good.stats()["it"] > 0
     s.finalize()
     good.finalize()
+
+
+def test_nothing_is_written_of_a_failed_step(make_case, monkeypatch):
+    import os
+
+    pkg = package()
+    spec, mesh, d, U0, prof = make_case("tiny-sor", n=(64, 40, 40), dt=1e-4, output_start_time=0.0,
+                                        output_interval_time=1e-4, probes=[[5.0, 2.5, 1.0]])
+    monkeypatch.setenv("DALM_BARRIER_POLLS", "1")
+    s = pkg.Solver(d, write_output=True)
+    s.set_state(U0)
+    s.step(1)
+    out = os.path.join(d, "output")
+    before = sorted(os.listdir(out))
+    with pytest.raises(pkg.DalmError) as e:
+        s.step(3)
+    assert e.value.code == 5
+    assert sorted(os.listdir(out)) == before
+    s.finalize()
+    with open(os.path.join(out, "probe0.csv")) as f:
+        assert len([r for r in f if r[0].isdigit()]) == 1  # step 0
