@@ -890,15 +890,16 @@ struct dalm_handle {
         }
     }
     // The reference's solve (FP64) from the current p; `used` iterations of
-    // the case's cap are already spent.
-    void solve_fp64(long long used) {
+    // the case's cap are already spent.  ahead: the caller does not need the
+    // solve's state (h_kst[0]) on return.
+    void solve_fp64(long long used, bool ahead = false) {
         double ncell = (double)g.ni() * g.nj() * g.nk();
         launch_poisson_begin(L, d_kst, max_it - used, tol, ncell);
         if (pcfg.method == PM_BICG)
             launch_bicg_init(L, g, coef, pb, pcfg, Partials<1>{partial, ticket}, d_kst);
         // a resident solve that ends within one launch needs no answer here:
         // the step goes on, and its statistics come with the next ones read
-        states_ahead = resident && !mixed && !trace && max_it - used <= RESIDENT_BUDGET;
+        states_ahead = ahead && resident && !trace && max_it - used <= RESIDENT_BUDGET;
         if (states_ahead) {
             launch_resident_solve(L, g, coef, pb, pcfg, RESIDENT_BUDGET, partial, d_sync, d_kst);
             return;
@@ -911,7 +912,7 @@ struct dalm_handle {
     void stage_poisson() {
         StageTimer t(this, DALM_STAGE_POISSON);
         if (!mixed) {
-            solve_fp64(0);
+            solve_fp64(0, true);
         } else {
             solve_mixed();
         }
