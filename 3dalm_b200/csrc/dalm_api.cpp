@@ -468,15 +468,15 @@ struct dalm_handle {
     // 128x64x64, 164 / 113 on 384x192x100; Jacobi 118 / 75 there; BiCGStab
     // 74 / 29 on 100x40x33, 93 / 58 on 131x75x53).  Larger Jacobi(3)-BiCGStab
     // solves run as fused half-iterations (192x96x64: 125 / 107, 512x256x128:
-    // 860 / 680).  fused_krylov and fused_jacobi ask for a launched form, and
-    // profiling times launches, so it keeps the kernel-per-loop form of small
-    // grids.
+    // 860 / 680).  fused_krylov and fused_jacobi ask for a launched form;
+    // profiling times launches and a trace of batches reads the residual
+    // between them, so both keep the kernel-per-loop form of small grids.
     void choose_route() {
         int coop = 0;
         DALM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, opt.device));
         const bool holds = coop && resident_available(pcfg, g);
         fused = fused_bicg_available(pcfg) && !opt.fused_jacobi && (opt.fused_krylov || !holds);
-        resident = holds && !opt.fused_krylov && !opt.fused_jacobi && !opt.profile;
+        resident = holds && !opt.fused_krylov && !opt.fused_jacobi && !opt.profile && !trace_batches;
     }
 
     // The multigrid levels of the inner solves (multigrid.cuh): merged-cell
