@@ -474,9 +474,16 @@ struct dalm_handle {
     void choose_route() {
         int coop = 0;
         DALM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, opt.device));
+        // (plans for another number of multiprocessors than the device reports)
+        if (const char *n = std::getenv("DALM_SM_COUNT"))
+            pcfg.sm_count = (int)std::min<long long>(L.blocks, std::max<long long>(1, std::atoll(n)));
         const bool holds = coop && resident_available(pcfg, g);
-        fused = fused_bicg_available(pcfg) && !opt.fused_jacobi && (opt.fused_krylov || !holds);
+        choose_launched(holds);
         resident = holds && !opt.fused_krylov && !opt.fused_jacobi && !opt.profile && !trace_batches;
+    }
+
+    void choose_launched(bool small) {
+        fused = fused_bicg_available(pcfg) && !opt.fused_jacobi && (opt.fused_krylov || !small);
     }
 
     // The multigrid levels of the inner solves (multigrid.cuh): merged-cell
@@ -880,14 +887,24 @@ struct dalm_handle {
         }
         return h_kst[which].it;
     }
-    // the same loop for a resident solve: returns its iterations
-    long long run_resident(long long cap) {
-        for (long long issued = 0;; issued += RESIDENT_BUDGET) {
+    // one launch of a resident solve; false when the device refuses it, and
+    // this handle's solves are launched from then on
+    bool enqueue_resident() {
+        if (launch_resident_solve(L, g, coef, pb, pcfg, RESIDENT_BUDGET, partial, d_sync, d_kst)) return true;
+        resident = false;
+        choose_launched(false);
+        return false;
+    }
+    // FP64 solve from the state that launch_poisson_begin (and
+    // launch_bicg_init) set up: its iterations
+    long long run_fp64(long long hint, long long cap) {
+        for (long long issued = 0; resident; issued += RESIDENT_BUDGET) {
             if (issued > cap) throw std::runtime_error("Poisson loop did not stop at its iteration limit");
-            launch_resident_solve(L, g, coef, pb, pcfg, RESIDENT_BUDGET, partial, d_sync, d_kst);
+            if (!enqueue_resident()) break;
             fetch_states();
             if (h_kst[0].done) return h_kst[0].it;
         }
+        return run_batches(0, hint, cap);
     }
     // The reference's solve (FP64) from the current p; `used` iterations of
     // the case's cap are already spent.  ahead: the caller does not need the
@@ -901,11 +918,10 @@ struct dalm_handle {
         // the step goes on, and its statistics come with the next ones read
         states_ahead = ahead && resident && !trace && max_it - used <= RESIDENT_BUDGET;
         if (states_ahead) {
-            launch_resident_solve(L, g, coef, pb, pcfg, RESIDENT_BUDGET, partial, d_sync, d_kst);
-            return;
+            if (enqueue_resident()) return;
+            states_ahead = false;
         }
-        long long hint = mixed ? refine_fp64_it : last_it;
-        long long n = resident ? run_resident(max_it - used) : run_batches(0, hint, max_it - used);
+        long long n = run_fp64(mixed ? refine_fp64_it : last_it, max_it - used);
         refine_fp64_it = n;
         h_kst[0].it = used + n;
     }
@@ -1640,7 +1656,7 @@ struct dalm_handle {
         launch_poisson_begin(L, d_kst, max_it, tol_abs, ncell);
         if (pcfg.method == PM_BICG)
             launch_bicg_init(L, g, coef, pb, pcfg, Partials<1>{partial, ticket}, d_kst);
-        long long n = resident ? run_resident(max_it) : run_batches(0, adj_hint > 0 ? adj_hint : last_it, max_it);
+        long long n = run_fp64(adj_hint > 0 ? adj_hint : last_it, max_it);
         adj_hint = n;
         return n;
     }

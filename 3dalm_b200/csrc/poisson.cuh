@@ -132,8 +132,9 @@ void launch_bicg_iteration_fused(const LaunchCtx &L, const Grid &g, const Poisso
 bool resident_available(const PoissonConfig &cfg, const Grid &g);
 // Up to `budget` iterations of the solve that launch_poisson_begin (and
 // launch_bicg_init) set up, or of the one an earlier launch left unfinished.
-// part: four doubles of device memory per SM; sync: two words.
-void launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
+// part: four doubles of device memory per SM; sync: two words.  false: the
+// device cannot hold the solve's blocks together, and nothing was launched.
+bool launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
                            const PoissonBufs &B, const PoissonConfig &cfg, long long budget,
                            double *part, unsigned *sync, KrylovState *st);
 

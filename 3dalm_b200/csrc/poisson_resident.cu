@@ -872,13 +872,22 @@ k_resident_bicg_sor(Grid g, PoissonCoef C, Cells cells, PoissonBufs B, int sweep
 // per plane.
 constexpr size_t AXIS_SMEM = 200 * 1024, PACKED_SMEM = 150 * 1024, RESIDENT_SMEM = 208 * 1024;
 
+// false when the device does not hold the blocks together after all (it can
+// have fewer multiprocessors to give than it reports): nothing was launched
 template <typename K, typename... Args>
-void cooperative(const LaunchCtx &L, K kernel, int blocks, int threads, size_t smem, Args... args) {
+bool cooperative(const LaunchCtx &L, K kernel, int blocks, int threads, size_t smem, Args... args) {
     void *ptrs[] = {(void *)&args...};
     allow_shared(kernel, RESIDENT_SMEM);
     L.pre(KK_RESIDENT);
-    DALM_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(blocks), dim3(threads), ptrs, smem, L.s));
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel((const void *)kernel, dim3(blocks), dim3(threads), ptrs, smem, L.s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return false;
+    }
+    DALM_CUDA(e);
     L.post(KK_RESIDENT);
+    return true;
 }
 
 template <int U, bool MEM>
@@ -886,10 +895,8 @@ bool resident_bicg(const LaunchCtx &L, const Grid &g, const PoissonCoef &C, cons
                    const PoissonConfig &cfg, long long budget, double *part, unsigned *sync,
                    KrylovState *st) {
     const Columns Q = Columns::make(cfg.seg.box, U);
-    if (Q.threads > (unsigned)cfg.sm_count * RT) return false;
-    cooperative(L, k_resident_bicg<U, MEM>, (int)((Q.threads + RT - 1) / RT), RT,
-                3 * sizeof(double) * (size_t)(g.ni() + U), g, C, Q, B, budget, part, sync, cfg.wait_polls, st);
-    return true;
+    return cooperative(L, k_resident_bicg<U, MEM>, (int)((Q.threads + RT - 1) / RT), RT,
+                       3 * sizeof(double) * (size_t)(g.ni() + U), g, C, Q, B, budget, part, sync, cfg.wait_polls, st);
 }
 
 }  // namespace
@@ -907,19 +914,19 @@ bool resident_available(const PoissonConfig &cfg, const Grid &g) {
            AxisCoef::bytes(g) <= AXIS_SMEM;
 }
 
-void launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
+bool launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
                            const PoissonBufs &B, const PoissonConfig &cfg, long long budget,
                            double *part, unsigned *sync, KrylovState *st) {
     const Cells cells = Cells::make(cfg.seg.box);
+    const unsigned threads = (unsigned)cfg.sm_count * RT;
     DALM_CUDA(cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), L.s));
     if (cfg.method == PM_BICG && cfg.pc == PC_JACOBI) {
         // the fewest planes per thread that fit the grid on the device
-        if (!resident_bicg<1, false>(L, g, C, B, cfg, budget, part, sync, st) &&
-            !resident_bicg<2, false>(L, g, C, B, cfg, budget, part, sync, st) &&
-            !resident_bicg<4, false>(L, g, C, B, cfg, budget, part, sync, st) &&
-            !resident_bicg<8, true>(L, g, C, B, cfg, budget, part, sync, st))
-            throw std::logic_error("grid too large for the resident BiCGStab");
-        return;
+        auto fits = [&](int planes) { return Columns::make(cfg.seg.box, planes).threads <= threads; };
+        if (fits(1)) return resident_bicg<1, false>(L, g, C, B, cfg, budget, part, sync, st);
+        if (fits(2)) return resident_bicg<2, false>(L, g, C, B, cfg, budget, part, sync, st);
+        if (fits(4)) return resident_bicg<4, false>(L, g, C, B, cfg, budget, part, sync, st);
+        return resident_bicg<8, true>(L, g, C, B, cfg, budget, part, sync, st);
     }
     // a grid of up to 8192 cells in one block, which needs no grid barrier;
     // else two cells of a colour per thread, at most a block per SM
@@ -929,24 +936,21 @@ void launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef 
     if (cfg.method == PM_SOR) {
         const Packed Q = Packed::make(cfg.seg.box);
         const size_t axis = 3 * sizeof(double) * (size_t)(Q.ni + SOR_UI), packed = 2 * sizeof(double) * (size_t)Q.total();
-        if (Q.threads <= RT && packed <= PACKED_SMEM) {
-            cooperative(L, k_resident_sor_regs<true>, 1, RT, axis + packed, g, C, cfg.seg.box, Q, B.x, B.tp, B.ts, B.b,
-                        cfg.relax, budget, part, sync, cfg.wait_polls, st);
-            return;
-        }
-        if (Q.threads <= (unsigned)cfg.sm_count * RT) {
-            cooperative(L, k_resident_sor_regs<false>, (int)((Q.threads + RT - 1) / RT), RT, axis, g, C, cfg.seg.box,
-                        Q, B.x, B.tp, B.ts, B.b, cfg.relax, budget, part, sync, cfg.wait_polls, st);
-            return;
-        }
-        cooperative(L, k_resident_sor, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, cfg.relax, budget,
-                    part, sync, cfg.wait_polls, st);
-    } else if (cfg.method == PM_JACOBI)
-        cooperative(L, k_resident_jacobi, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, budget, part,
-                    sync, cfg.wait_polls, st);
-    else
-        cooperative(L, k_resident_bicg_sor, blocks, RT, smem, g, C, cells, B, cfg.pc_sweeps, cfg.pc_relax,
-                    budget, part, sync, cfg.wait_polls, st);
+        if (Q.threads <= RT && packed <= PACKED_SMEM)
+            return cooperative(L, k_resident_sor_regs<true>, 1, RT, axis + packed, g, C, cfg.seg.box, Q, B.x, B.tp,
+                               B.ts, B.b, cfg.relax, budget, part, sync, cfg.wait_polls, st);
+        if (Q.threads <= threads)
+            return cooperative(L, k_resident_sor_regs<false>, (int)((Q.threads + RT - 1) / RT), RT, axis, g, C,
+                               cfg.seg.box, Q, B.x, B.tp, B.ts, B.b, cfg.relax, budget, part, sync, cfg.wait_polls,
+                               st);
+        return cooperative(L, k_resident_sor, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, cfg.relax, budget,
+                           part, sync, cfg.wait_polls, st);
+    }
+    if (cfg.method == PM_JACOBI)
+        return cooperative(L, k_resident_jacobi, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, budget, part,
+                           sync, cfg.wait_polls, st);
+    return cooperative(L, k_resident_bicg_sor, blocks, RT, smem, g, C, cells, B, cfg.pc_sweeps, cfg.pc_relax,
+                       budget, part, sync, cfg.wait_polls, st);
 }
 
 }  // namespace dalm
