@@ -898,11 +898,11 @@ struct dalm_handle {
     // FP64 solve from the state that launch_poisson_begin (and
     // launch_bicg_init) set up: its iterations
     long long run_fp64(long long hint, long long cap) {
-        for (long long issued = 0; resident; issued += RESIDENT_BUDGET) {
-            if (issued > cap) throw std::runtime_error("Poisson loop did not stop at its iteration limit");
+        for (long long issued = RESIDENT_BUDGET; resident; issued += RESIDENT_BUDGET) {
             if (!enqueue_resident()) break;
             fetch_states();
             if (h_kst[0].done) return h_kst[0].it;
+            if (issued > cap) throw std::runtime_error("Poisson loop did not stop at its iteration limit");
         }
         return run_batches(0, hint, cap);
     }

@@ -56,3 +56,15 @@ def test_cluster_route(make_case, n):
         count.append(s.timings()[1])
         s.finalize()
     assert count[0] < 0.6 * count[1], count
+
+
+@pytest.mark.parametrize("name", ["tiny-sor", "tiny-jacobi", "tiny-bicg", "tiny-sorpc"])
+@pytest.mark.parametrize("cap", [-1500, -1, 0, 1])
+def test_smallest_caps(make_case, monkeypatch, capfd, name, cap):
+    """A loop tests its cap after an iteration, so one is always done: launched,
+    resident, and resident with the host waiting for it (a trace)."""
+    its = []
+    for options, trace in (({"profile": True}, "0"), ({}, "0"), ({}, "1")):
+        monkeypatch.setenv("DALM_TRACE_POISSON", trace)
+        its.append(solve(make_case, name, (24, 12, 12), cap, **options)[0][0])
+    assert its == [1, 1, 1]
