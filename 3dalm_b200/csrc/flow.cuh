@@ -93,18 +93,48 @@ __device__ inline void warp_serial_sums(const Grid &g, Term term, double (&total
             }
 }
 
+// Outside {0} and 2^LO <= |a| < 2^HI (infinities and NaN among them).
+template <int LO, int HI>
+__device__ __forceinline__ bool is_far(double a) {
+    constexpr unsigned lo = (unsigned)(1023 + LO) << 20, hi = (unsigned)(1023 + HI) << 20;
+    return ((unsigned)__double2hiint(a) & 0x7fffffffu) - lo >= hi - lo && a != 0.0;
+}
+
 // a / b with IEEE rounding, from y = 1 / b rounded to nearest (Markstein, IBM
 // J. Res. Dev. 34 (1990): with y the correctly rounded reciprocal and q
 // within one unit of a / b, q + (a - b q) y rounds to the correctly rounded
 // quotient; the first correction brings a y within one unit).  Five FP64
 // operations against the fourteen or so and the branch of a division.  b is a
-// mesh spacing or volume.  The remainders are exact for a = 0 and from
-// |a| = 2^-900 up; below that the quotient may be two units off, and an
-// infinite a gives NaN (the step reports either as a non-finite state).
-__device__ __forceinline__ double div_by(double a, double b, double y) {
+// mesh spacing or volume, 2^-100 to 2^100.  The remainders are exact for a = 0
+// and from |a| = 2^-968 up, and the quotient is finite below 2^900.
+__device__ __forceinline__ double div_near(double a, double b, double y) {
     const double q0 = a * y;
     const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
     return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+// the N quotients a / b, every a: one test for all of them, in integers
+template <int N>
+__device__ __forceinline__ void divs_by(double (&a)[N], const double (&b)[N], const double (&y)[N]) {
+    constexpr unsigned lo = (unsigned)(1023 - 900) << 20, hi = (unsigned)(1023 + 900) << 20;
+    unsigned most = 0;
+#pragma unroll
+    for (int n = 0; n < N; n++) most = max(most, ((unsigned)__double2hiint(a[n]) & 0x7fffffffu) - lo);
+    bool far = false;
+    if (most >= hi - lo)  // a zero, or far
+#pragma unroll
+        for (int n = 0; n < N; n++) far |= is_far<-900, 900>(a[n]);
+    if (far) {
+#pragma unroll
+        for (int n = 0; n < N; n++) a[n] = a[n] / b[n];
+    } else {
+#pragma unroll
+        for (int n = 0; n < N; n++) a[n] = div_near(a[n], b[n], y[n]);
+    }
+}
+// the same for every a
+static __device__ __noinline__ double div_far(double a, double b) { return a / b; }
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    return is_far<-900, 900>(a) ? div_far(a, b) : div_near(a, b, y);
 }
 
 // The cells of the face box (the interior and one layer below it per axis)

@@ -5,6 +5,7 @@
 // the reference bit for bit; the only libm call is cbrt in the eddy
 // viscosity.
 #include <algorithm>
+#include <type_traits>
 
 #include "flow.cuh"
 
@@ -121,10 +122,15 @@ __device__ __forceinline__ bool interior(const Grid &g, int i, int j, int k) {
 // cell is the next plane's west face and is carried; the y and z faces are
 // computed by both cells, which share half of their limiter terms.
 //
+// Quotients by spacings are div_near's while every value that the block has
+// loaded lies in its range, which a thread tests for the values it loads
+// (a branch in every quotient: 1.75 ms on 512 x 256 x 128, this 1.25); else
+// divisions.
+//
 // Bound by FP64 issue and latency (its bytes would take 0.25 ms on
-// 512 x 256 x 128; the FP64 pipe is 47 % busy).  There: 1.32 ms, against 3.40 ms with 36 divisions a cell, six limiter terms per
-// face pair through fmin / fmax, and every neighbour loaded through 64-bit
-// indices.
+// 512 x 256 x 128; the FP64 pipe is 47 % busy).  There: 1.25 ms, against
+// 3.40 ms with 36 divisions a cell, six limiter terms per face pair through
+// fmin / fmax, and every neighbour loaded through 64-bit indices.
 constexpr int PR = TJ + 4, PCOL = TK + 4;  // plane with halo: 12 x 36
 template <int LIM>
 __global__ void __launch_bounds__(TILE_THREADS, 2)
@@ -185,7 +191,18 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
         if (hrow >= 0) plane[0][m][hrow][hcol] = V.c[m][hc];
     }
     const double rre = 1 / P.re;
-    __syncthreads();
+    // far: a value that the block has loaded is neither 0 nor within 2^-760 to
+    // 2^200.  Without one, differences of values are 0 or at least 2^-812, and
+    // differences of their quotients by spacings within 2^-100 to 2^100 at
+    // least 2^-965: div_near's range.
+    bool far = false;
+#pragma unroll
+    for (int m = 0; m < 3; m++) {
+#pragma unroll
+        for (int d = 0; d < 5; d++) far |= is_far<-760, 200>(ring[m][d]);
+        if (hrow >= 0) far |= is_far<-760, 200>(plane[0][m][hrow][hcol]);
+    }
+    far = __syncthreads_or(far);
     for (int i = i0; i < i1; i++) {
         const int b = (i - i0) & 1, c = c0 + (i - i0) * sx;
         const bool more = i + 1 < i1;
@@ -200,7 +217,9 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
             }
             cp_async_commit();
         }
-        if (valid) {
+        auto cell = [&](auto exact) {
+            constexpr bool EX = decltype(exact)::value;
+            auto quot = [](double a, double d, double y) { return EX ? a / d : div_near(a, d, y); };
             const double JE = JU.c[0][c], JN = JU.c[1][c], JS = JU.c[1][c - sy], JT = JU.c[2][c],
                          JB = JU.c[2][c - 1], filter = P.filter2[c];
             const double dx = P.m.dx[i], idx = P.invd[0][i];
@@ -214,9 +233,9 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
 #pragma unroll
                 for (int m = 0; m < 3; m++) {
                     const double(*t)[PCOL] = plane[b][m];
-                    G[m][0] = div_by(ring[m][3] - ring[m][1], xe - xw, ix.y);
-                    G[m][1] = div_by(t[row + 3][lane + 2] - t[row + 1][lane + 2], ya[CC][row], ya[RCC][row]);
-                    G[m][2] = div_by(t[row + 2][lane + 3] - t[row + 2][lane + 1], za[CC][lane], za[RCC][lane]);
+                    G[m][0] = quot(ring[m][3] - ring[m][1], xe - xw, ix.y);
+                    G[m][1] = quot(t[row + 3][lane + 2] - t[row + 1][lane + 2], ya[CC][row], ya[RCC][row]);
+                    G[m][2] = quot(t[row + 2][lane + 3] - t[row + 2][lane + 1], za[CC][lane], za[RCC][lane]);
                 }
                 const double s1 = 2 * sq(G[0][0]), s2 = 2 * sq(G[1][1]), s3 = 2 * sq(G[2][2]);
                 const double s4 = sq(G[0][1] + G[1][0]), s5 = sq(G[0][2] + G[2][0]),
@@ -246,14 +265,18 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
                 const double conv = div_by(fE - fW[m] + fN - fS + fT - fB, J, iJ);
                 fW[m] = fE;
                 const double diff =
-                    visc * (div_by(div_by(e1, xe - xi, ix.x) - div_by(w1, xi - xw, ixW), dx, idx) +
-                            div_by(div_by(n1, ya[UP][row], ya[RUP][row]) -
-                                       div_by(s1, ya[DN][row], ya[RDN][row]), dy, ya[RD][row]) +
-                            div_by(div_by(t1, za[UP][lane], za[RUP][lane]) -
-                                       div_by(b1, za[DN][lane], za[RDN][lane]), dz, za[RD][lane]));
+                    visc * (quot(quot(e1, xe - xi, ix.x) - quot(w1, xi - xw, ixW), dx, idx) +
+                            quot(quot(n1, ya[UP][row], ya[RUP][row]) -
+                                       quot(s1, ya[DN][row], ya[RDN][row]), dy, ya[RD][row]) +
+                            quot(quot(t1, za[UP][lane], za[RUP][lane]) -
+                                       quot(b1, za[DN][lane], za[RDN][lane]), dz, za[RD][lane]));
                 const double fm = has_f ? F.c[m][c] : 0.0;
                 Un.c[m][c] = fc + P.dt * (-conv + diff + fm);
             }
+        };
+        if (valid) {
+            if (far) cell(std::true_type{});
+            else cell(std::false_type{});
             // the guide cells at the ends of this k row (U* = U^n there)
             if (k == g.gc || k == g.nz - g.gc - 1) {
                 const int d = k == g.gc ? -1 : 1;
@@ -273,8 +296,13 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
                 ring[m][4] = nxt[m];
             }
             cp_async_wait<0>();
+#pragma unroll
+            for (int m = 0; m < 3; m++) {
+                far |= is_far<-760, 200>(nxt[m]);
+                if (hrow >= 0) far |= is_far<-760, 200>(plane[b ^ 1][m][hrow][hcol]);
+            }
         }
-        __syncthreads();
+        far = __syncthreads_or(far);
     }
 }
 
@@ -340,7 +368,7 @@ __device__ __forceinline__ double face_z(const StepParams &P, Vec3<const double>
 // Covers faces i,j,k in [gc-1, N-gc).  Blocks [0, T.count) march the
 // interior's column segments along i, carrying the west face and the centre
 // velocity; the RHS's south and bottom faces are recomputed (same
-// arithmetic, same bits).  512 x 256 x 128: 0.22 ms, 4.3 TB/s (0.40 ms over
+// arithmetic, same bits).  512 x 256 x 128: 0.21 ms, 4.4 TB/s (0.40 ms over
 // the face box, every face from scratch).
 template <bool RHS>
 __global__ void __launch_bounds__(TILE_THREADS)
@@ -474,7 +502,7 @@ __device__ __forceinline__ double proj_face(const StepParams &P, Vec3<double> JU
 // A thread owns the three faces of its lower cell; the divergence of an
 // interior cell also needs its west face, carried along the march, and its
 // south and bottom faces, which it recomputes from the pre-projection flux.
-// 512 x 256 x 128: 0.56 ms, 3.1 TB/s (0.95 ms over the face box, with eleven
+// 512 x 256 x 128: 0.52 ms, 3.4 TB/s (0.95 ms over the face box, with eleven
 // divisions a cell and the west face recomputed).
 // Because other threads overwrite those faces in the same launch, the
 // projected flux goes to a second buffer (JUout) and the host swaps the two.
@@ -516,15 +544,19 @@ k_project(StepParams P, Segments T, Vec3<double> U, Vec3<double> JUin, Vec3<doub
             double u = U.c[0][c], v = U.c[1][c], w = U.c[2][c];
             const double dx = P.m.dx[i], xz = dx * dz, xy = dx * dy;
             const double2 ix = P.inv[0][i];
-            const double fe = ju - dt * yz * div_by(pe - pc, P.m.x[i + 1] - P.m.x[i], ix.x);
-            const double fn = wall_n ? 0.0 : jv - dt * xz * div_by(pn - pc, yN, iy.x);
-            const double ft = wall_t ? 0.0 : jw - dt * xy * div_by(pt - pc, zT, iz.x);
+            double q[8] = {pe - pc, pn - pc, pt - pc, pc - ps, pc - pb, dt * (pe - pw), dt * (pn - ps), dt * (pt - pb)};
+            const double by[8] = {P.m.x[i + 1] - P.m.x[i], yN, zT, yS, zB, P.m.x[i + 1] - P.m.x[i - 1], yC, zC};
+            const double rb[8] = {ix.x, iy.x, iz.x, iyS, izB, ix.y, iy.y, iz.y};
+            divs_by(q, by, rb);
+            const double fe = ju - dt * yz * q[0];
+            const double fn = wall_n ? 0.0 : jv - dt * xz * q[1];
+            const double ft = wall_t ? 0.0 : jw - dt * xy * q[2];
             JUout.c[0][c] = fe;
             JUout.c[1][c] = fn;
             JUout.c[2][c] = ft;
-            u = u - div_by(dt * (pe - pw), P.m.x[i + 1] - P.m.x[i - 1], ix.y);
-            v = v - div_by(dt * (pn - ps), yC, iy.y);
-            w = w - div_by(dt * (pt - pb), zC, iz.y);
+            u = u - q[5];
+            v = v - q[6];
+            w = w - q[7];
             if (P.solid) {  // set_solid_U (src/cfd.h:1143-1160)
                 const double sf = P.solid[c];
                 u = (1. - sf) * u;
@@ -534,13 +566,14 @@ k_project(StepParams P, Segments T, Vec3<double> U, Vec3<double> JUin, Vec3<doub
             U.c[0][c] = u;
             U.c[1][c] = v;
             U.c[2][c] = w;
-            const double fs = wall_s ? 0.0 : jvs - dt * xz * div_by(pc - ps, yS, iyS);
-            const double fb = wall_b ? 0.0 : jwb - dt * xy * div_by(pc - pb, zB, izB);
+            const double fs = wall_s ? 0.0 : jvs - dt * xz * q[3];
+            const double fb = wall_b ? 0.0 : jwb - dt * xy * q[4];
             const double J = dx * dy * dz;
             const double d = (fe - fw + fn - fs + ft - fb) / J;
             div2 += d * d;
-            const double local = div_by(fabs(u) * dt, dx, P.invd[0][i]) + div_by(fabs(v) * dt, dy, idy) +
-                                 div_by(fabs(w) * dt, dz, idz);
+            double co[3] = {fabs(u) * dt, fabs(v) * dt, fabs(w) * dt};
+            divs_by(co, {dx, dy, dz}, {P.invd[0][i], idy, idz});
+            const double local = co[0] + co[1] + co[2];
             cfl = local > cfl ? local : cfl;
             fw = fe;
             pw = pc;

@@ -423,7 +423,7 @@ k_flux32(StepParams P, Segments T, MixedGeom Gm, Vec3<const float> U, Vec3<float
 // Blocks [0, T.count) march the interior's column segments with plane i + 1's
 // operands loaded before plane i is computed, the others take the faces below
 // the interior.  Bound by memory latency and FP64 issue: three blocks per SM.
-// 512x256x128: 353 us, against 401 us over the face box with four
+// 512x256x128: 343 us, against 401 us over the face box with four
 // divisions a cell.
 struct ProjectOps {
     double pe, pn, ps, pt, pb;    // p at i + 1, j +- 1, k +- 1
