@@ -28,8 +28,14 @@ __device__ __forceinline__ double va_switch(double a, double b) {
 
 // The b = (3 - kappa) / (1 - kappa) limiter term s_a max(0, min(|a|, s_a bb b))
 // (src/cfd.h:37-54) from a and t = bb b: the smaller of the two if they have
-// the same sign, else 0.
+// the same sign, else 0.  EX: also where one of them is NaN, which the
+// reference's minimum ignores.
+template <bool EX>
 __device__ __forceinline__ double limited(double a, double t) {
+    if (EX) {
+        const double s = sgn(a);
+        return s * fmax(0., fmin(fabs(a), s * t));
+    }
     const double m = fabs(t) < fabs(a) ? t : a;
     return (__double2hiint(a) ^ __double2hiint(t)) >= 0 ? m : 0.0;
 }
@@ -39,7 +45,7 @@ __device__ __forceinline__ double limited(double a, double t) {
 // and the upwind flux (src/cfd.h:37-60).  The reference forms a face's states
 // once for each of the two cells; they are the same operations on the same
 // values, so computing the face once gives both cells' bits.
-template <int LIM>
+template <int LIM, bool EX>
 __device__ __forceinline__ double face_flux(double fc, double fp, double d2, double d3, double d4,
                                             double J) {
     const double kap = 1. / 3.;
@@ -51,8 +57,8 @@ __device__ __forceinline__ double face_flux(double fc, double fp, double d2, dou
         l = fc + (sc / 4.) * ((1. - kap * sc) * d2 + (1. + kap * sc) * d3);
     } else {
         const double t2 = bb * d2, t3 = bb * d3, t4 = bb * d4;
-        const double g6 = limited(d4, t3), g5 = limited(d3, t4);
-        const double g4 = limited(d3, t2), g3 = limited(d2, t3);
+        const double g6 = limited<EX>(d4, t3), g5 = limited<EX>(d3, t4);
+        const double g4 = limited<EX>(d3, t2), g3 = limited<EX>(d2, t3);
         r = fp - 0.25 * ((1. - kap) * g6 + (1. + kap) * g5);
         l = fc + 0.25 * ((1. - kap) * g3 + (1. + kap) * g4);
     }
@@ -124,11 +130,11 @@ __device__ __forceinline__ bool interior(const Grid &g, int i, int j, int k) {
 //
 // Quotients by spacings are div_near's while every value that the block has
 // loaded lies in its range, which a thread tests for the values it loads
-// (a branch in every quotient: 1.75 ms on 512 x 256 x 128, this 1.25); else
+// (a branch in every quotient: 1.75 ms on 512 x 256 x 128, this 1.23); else
 // divisions.
 //
 // Bound by FP64 issue and latency (its bytes would take 0.25 ms on
-// 512 x 256 x 128; the FP64 pipe is 47 % busy).  There: 1.25 ms, against
+// 512 x 256 x 128; the FP64 pipe is 47 % busy).  There: 1.23 ms, against
 // 3.40 ms with 36 divisions a cell, six limiter terms per face pair through
 // fmin / fmax, and every neighbour loaded through 64-bit indices.
 constexpr int PR = TJ + 4, PCOL = TK + 4;  // plane with halo: 12 x 36
@@ -177,14 +183,6 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
     };
     if (lane == 0 && j < T.box.hi[1]) axis(1, P.m.y, P.m.dy, j, &ya[0][row], TJ);
     if (row == 0 && k < T.box.hi[2]) axis(2, P.m.z, P.m.dz, k, &za[0][lane], TK);
-    double fW[3] = {0, 0, 0};
-    if (valid) {
-        const double JUW = JU.c[0][c0 - sx];
-#pragma unroll
-        for (int m = 0; m < 3; m++)
-            fW[m] = face_flux<LIM>(ring[m][1], ring[m][2], ring[m][1] - ring[m][0],
-                                   ring[m][2] - ring[m][1], ring[m][3] - ring[m][2], JUW);
-    }
 #pragma unroll
     for (int m = 0; m < 3; m++) {
         plane[0][m][row + 2][lane + 2] = ring[m][2];
@@ -203,6 +201,16 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
         if (hrow >= 0) far |= is_far<-760, 200>(plane[0][m][hrow][hcol]);
     }
     far = __syncthreads_or(far);
+    double fW[3] = {0, 0, 0};
+    if (valid) {
+        const double JUW = JU.c[0][c0 - sx];
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            const double d2 = ring[m][1] - ring[m][0], d3 = ring[m][2] - ring[m][1], d4 = ring[m][3] - ring[m][2];
+            fW[m] = far ? face_flux<LIM, true>(ring[m][1], ring[m][2], d2, d3, d4, JUW)
+                        : face_flux<LIM, false>(ring[m][1], ring[m][2], d2, d3, d4, JUW);
+        }
+    }
     for (int i = i0; i < i1; i++) {
         const int b = (i - i0) & 1, c = c0 + (i - i0) * sx;
         const bool more = i + 1 < i1;
@@ -257,11 +265,11 @@ k_predict(StepParams P, Segments T, Vec3<const double> V, Vec3<double> Un, Vec3<
                              s2 = ys - t[row][lane + 2];
                 const double t1 = zt - fc, t2 = t[row + 2][lane + 4] - zt, b1 = fc - zb,
                              b2 = zb - t[row + 2][lane];
-                const double fE = face_flux<LIM>(fc, ring[m][3], w1, e1, ring[m][4] - ring[m][3], JE);
-                const double fN = face_flux<LIM>(fc, yn, s1, n1, n2, JN);
-                const double fS = face_flux<LIM>(ys, fc, s2, s1, n1, JS);
-                const double fT = face_flux<LIM>(fc, zt, b1, t1, t2, JT);
-                const double fB = face_flux<LIM>(zb, fc, b2, b1, t1, JB);
+                const double fE = face_flux<LIM, EX>(fc, ring[m][3], w1, e1, ring[m][4] - ring[m][3], JE);
+                const double fN = face_flux<LIM, EX>(fc, yn, s1, n1, n2, JN);
+                const double fS = face_flux<LIM, EX>(ys, fc, s2, s1, n1, JS);
+                const double fT = face_flux<LIM, EX>(fc, zt, b1, t1, t2, JT);
+                const double fB = face_flux<LIM, EX>(zb, fc, b2, b1, t1, JB);
                 const double conv = div_by(fE - fW[m] + fN - fS + fT - fB, J, iJ);
                 fW[m] = fE;
                 const double diff =

@@ -38,3 +38,32 @@ def test_stage_bits(make_case, scale):
         assert_identical(s, o, ("U", "JU", "p"), "project")
     s.finalize()
     o.close()
+
+
+@pytest.mark.parametrize("limiter", [0, 1])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_stage_bits_around_a_bad_cell(make_case, bad, limiter):
+    """What a cell that is not finite makes of its neighbours: the reference's
+    limiter takes the smaller of two differences and ignores one that is NaN."""
+    spec, mesh, d, U0, prof = make_case("tiny-sor", n=(40, 12, 40))
+    U, p = U0.copy(), np.random.default_rng(7).uniform(-1, 1, U0.shape[:3])
+    U[20, 8, 19, 1] = bad
+    U[30, 5, 35] = bad
+    p[12, 9, 30] = bad
+    s, o = package().Solver(d, reference_sums=True, limiter=limiter), O.CRestatement(d)
+    o.set_limiter(limiter)
+    for x in (s, o):
+        x.advance_clock()
+        x.set_state(U)
+        x.stage(0)
+    assert not np.all(np.isfinite(o.field("U")))
+    assert_identical(s, o, ("U",), "predict")
+    for x in (s, o):
+        x.stage(1)
+    assert_identical(s, o, ("JU", "b"), "flux_rhs")
+    for x in (s, o):
+        x.set_field("p", p)
+        x.stage(3)
+    assert_identical(s, o, ("U", "JU", "p"), "project")
+    s.finalize()
+    o.close()
