@@ -187,6 +187,14 @@ k_alm_project(StepParams P, AlmDev A, Box box, int ntk, int ntj, Vec3<FT> F) {
 }  // namespace
 
 template <typename T>
+void prepare_alm() {
+    allow_shared(k_alm_points<T>, ALM_SMEM);
+    allow_shared(k_alm_project<T>, ALM_SMEM);
+}
+template void prepare_alm<double>();
+template void prepare_alm<float>();
+
+template <typename T>
 void launch_alm_points(const LaunchCtx &L, const StepParams &P, const AlmDev &A, double t,
                        Vec3<const T> u) {
     if (A.ap_count <= 0) return;
@@ -194,7 +202,6 @@ void launch_alm_points(const LaunchCtx &L, const StepParams &P, const AlmDev &A,
     const size_t bytes = sizeof(double) * (2 * (size_t)A.ap_per_wt + P.g.nx + P.g.ny + P.g.nz + A.atk_count);
     const bool staged = bytes <= ALM_SMEM;
     const size_t smem = staged ? bytes : 0;
-    allow_shared(k_alm_points<T>, ALM_SMEM);
     const int threads = std::min(512, std::max(128, (A.ap_per_wt + 31) / 32 * 32));
     L.pre(KK_ALM_POINTS);
     k_alm_points<T><<<A.wt_count, threads, smem, L.s>>>(P, A, t, u, staged);
@@ -211,10 +218,8 @@ void launch_alm_project(const LaunchCtx &L, const StepParams &P, const AlmDev &A
     if (A.ap_count <= 0 || box.empty()) return;
     const int ntk = (box.hi[2] - box.lo[2] + TK - 1) / TK, ntj = (box.hi[1] - box.lo[1] + TJ - 1) / TJ;
     const int nti = (box.hi[0] - box.lo[0] + PP - 1) / PP;
-    // the list of points, beside 22 KB of static tables: with more than 6712
-    // points over the 48 KB that need no leave
+    // the list of points, beside 22 KB of static tables
     const size_t smem = sizeof(int) * (size_t)A.ap_count;
-    allow_shared(k_alm_project<FT>, ALM_SMEM);
     L.pre(KK_ALM_PROJECT);
     k_alm_project<FT><<<ntk * ntj * nti, TILE_THREADS, smem, L.s>>>(P, A, box, ntk, ntj, f);
     L.post(KK_ALM_PROJECT);

@@ -27,6 +27,9 @@ struct AlmDev {
     double *wt_torque, *wt_thrust;                  // outputs per turbine
 };
 
+// called once per handle before the launches below, on its device
+template <typename T>
+void prepare_alm();
 // update_ap_position + calc_ap_force (src/alm.h:233-414) and the per-turbine
 // sums (src/alm.h:384-398).
 // T: storage type of the sampled velocity (double, or float for the mixed

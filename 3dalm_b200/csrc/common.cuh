@@ -312,8 +312,9 @@ inline void pdl_launch(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t sme
 // Allows launches of `kernel` with up to `bytes` of dynamic shared memory.
 // The limit belongs to the function in the device's context, not to a handle,
 // and a launch above it fails: `bytes` is the most the kernel ever takes, the
-// same value on every call, so that no handle lowers the limit between another
-// one's call and launch.
+// same value on every call, so that no handle lowers the limit under another
+// one.  Called when a handle is set up (at every launch it cost 2 us of the
+// host's time).
 template <typename K>
 inline void allow_shared(K kernel, size_t bytes) {
     DALM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));

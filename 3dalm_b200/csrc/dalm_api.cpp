@@ -52,12 +52,10 @@ constexpr double INNER_RTOL = 1e-4;
 constexpr long long INNER_CAP = 100;
 constexpr double STALL = 0.85;
 constexpr long long MAX_REFINE = 1000;
-// Iterations per launch of a resident solve: bounds a launch to a fraction of a
-// second.
+// Iterations per launch of a resident solve.  A launch of the largest grids
+// that take one (25.6 M cells) lasts 0.3 s with SOR and 2.3 s with three sweeps
+// of the SOR preconditioner.
 constexpr long long RESIDENT_BUDGET = 1000;
-// Polls of one barrier wait of a resident solve, about a second; less by the
-// environment's DALM_BARRIER_POLLS.
-constexpr unsigned WAIT_POLLS = 1u << 21;
 // Adjoint pressure solves stop at this RMS residual relative to the RMS of
 // their right-hand side.
 constexpr double ADJ_RTOL = 1e-10;
@@ -376,9 +374,7 @@ struct dalm_handle {
         pcfg.reference_sums = opt.reference_sums ? 1 : 0;
         pcfg.jacobi2 = opt.fused_jacobi ? 1 : 0;
         pcfg.sm_count = sm_count;
-        pcfg.wait_polls = WAIT_POLLS;
-        if (const char *polls = std::getenv("DALM_BARRIER_POLLS"))
-            pcfg.wait_polls = (unsigned)std::min<long long>(WAIT_POLLS, std::max<long long>(1, std::atoll(polls)));
+        pcfg.stall_waits = std::getenv("DALM_STALL_BARRIERS") != nullptr;
         pcfg.seg = poisson_segments(g, sm_count);
         choose_route();
         // FP32 inner solves exist for BiCGStab only; SOR and Jacobi solves
@@ -461,12 +457,16 @@ struct dalm_handle {
     }
 
     // How an FP64 solve runs.  Whole, as one cooperative kernel, when that
-    // holds the grid (poisson_resident.cu: any SOR, Jacobi and SOR-preconditioned
-    // solve up to about 10 M cells, Jacobi(3)-BiCGStab up to eight cells a
-    // thread, 606,208 on 148 SMs): measured faster than a kernel per loop at
-    // every such size (us per iteration, launched / resident: SOR 26.3 / 7.3 on
-    // 128x64x64, 164 / 113 on 384x192x100; Jacobi 118 / 75 there; BiCGStab
-    // 74 / 29 on 100x40x33, 93 / 58 on 131x75x53).  Larger Jacobi(3)-BiCGStab
+    // holds the grid (poisson_resident.cu: SOR, Jacobi and SOR-preconditioned
+    // solves while cells * (nj + nk) < 2^32, the range of its index divisions,
+    // and the axes' tables fit shared memory, which is up to some 30 M cells;
+    // Jacobi(3)-BiCGStab up to eight cells a thread, 606,208 on 148 SMs):
+    // measured faster than a kernel per loop at every such size.  us per
+    // iteration, launched / resident: SOR 26.3 / 7.3 on 128x64x64, 139 / 87 on
+    // 384x192x100, 239 / 190 on 1000x128x128, 409 / 305 on 4000x80x80; Jacobi
+    // 93 / 50, 164 / 105 and 285 / 169 on the last three; SOR-preconditioned
+    // BiCGStab 903 / 637, 1555 / 1380 and 2620 / 2300; Jacobi(3)-BiCGStab
+    // 74 / 29 on 100x40x33, 93 / 58 on 131x75x53.  Larger Jacobi(3)-BiCGStab
     // solves run as fused half-iterations (192x96x64: 125 / 107, 512x256x128:
     // 860 / 680).  fused_krylov and fused_jacobi ask for a launched form;
     // profiling times launches and a trace of batches reads the residual
@@ -480,6 +480,7 @@ struct dalm_handle {
         const bool holds = coop && resident_available(pcfg, g);
         choose_launched(holds);
         resident = holds && !opt.fused_krylov && !opt.fused_jacobi && !opt.profile && !trace_batches;
+        if (resident) prepare_resident(pcfg);
     }
 
     void choose_launched(bool small) {
@@ -675,6 +676,8 @@ struct dalm_handle {
         alm.wt_count = (int)T;
         alm.ap_count = (int)cs.ap_count();
         if (alm.ap_count == 0) return;
+        if (f32) prepare_alm<float>();
+        else prepare_alm<double>();
         alm.ap_per_blade = (int)cs.ap_per_blade;
         alm.blades = (int)cs.blades;
         alm.ap_per_wt = (int)(cs.blades * cs.ap_per_blade);

@@ -290,7 +290,8 @@ struct KrylovState;
 // (256 cells); the mixed form then keeps its BiCGStab inner solves.
 bool mg_prepare(const MgDev &M);
 
-// false when no cluster of this size and shared memory fits the device
+// false when no cluster of this size and shared memory fits the device; called
+// before the first launch_mg_cluster
 bool mg_cluster_fits(const MgCluster &M);
 // x of level M.first = the V-cycle from that level on, of its f
 void launch_mg_cluster(const LaunchCtx &L, const MgCluster &M, const float *f, float *x,

@@ -378,13 +378,10 @@ cudaLaunchConfig_t config(const MgCluster &M, cudaLaunchAttribute *attr, cudaStr
     return cfg;
 }
 
-// the kernel for this cycle, with its shared memory and cluster size allowed
+// the kernel for this cycle
 auto kernel_of(const MgCluster &M) {
     const int R = (M.top.n[2] + 31) / 32;
-    auto k = R == 1 ? k_mg_cluster<1> : R == 2 ? k_mg_cluster<2> : R == 3 ? k_mg_cluster<3> : k_mg_cluster<4>;
-    allow_shared(k, MG_CLUSTER_SMEM);
-    DALM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    return k;
+    return R == 1 ? k_mg_cluster<1> : R == 2 ? k_mg_cluster<2> : R == 3 ? k_mg_cluster<3> : k_mg_cluster<4>;
 }
 
 }  // namespace
@@ -394,7 +391,10 @@ bool mg_cluster_fits(const MgCluster &M) {
     cudaLaunchConfig_t cfg = config(M, attr, 0);
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel_of(M), &cfg) != cudaSuccess) {
+    auto k = kernel_of(M);
+    allow_shared(k, MG_CLUSTER_SMEM);
+    DALM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

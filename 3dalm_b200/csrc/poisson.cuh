@@ -67,7 +67,7 @@ struct PoissonConfig {
     int reference_sums;  // 1: global sums in the reference's serial order
     int jacobi2;         // 1: FP64 Jacobi(3): the last two sweeps in one pass
     int sm_count;
-    unsigned wait_polls; // limit of a resident solve's barrier wait
+    bool stall_waits;    // a resident solve's barrier waits run out (tests)
     Segments seg;        // column segments of the interior (one per block)
     const MapTable *maps;
 };
@@ -130,6 +130,8 @@ void launch_bicg_iteration_fused(const LaunchCtx &L, const Grid &g, const Poisso
 // (poisson_resident.cu): SOR, Jacobi, BiCGStab with the Jacobi(3) or the SOR
 // preconditioner, not in the reference-order mode
 bool resident_available(const PoissonConfig &cfg, const Grid &g);
+// called once per handle before its first resident solve, on its device
+void prepare_resident(const PoissonConfig &cfg);
 // Up to `budget` iterations of the solve that launch_poisson_begin (and
 // launch_bicg_init) set up, or of the one an earlier launch left unfinished.
 // part: four doubles of device memory per SM; sync: two words.  false: the

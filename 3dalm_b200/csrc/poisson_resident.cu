@@ -22,15 +22,16 @@
 // What bounds them on grids that leave registers or L2 unfilled: the barriers
 // (1.24 us each) and the latency of the loads after them.  us per iteration,
 // launched / here: SOR 24x12x12 13.2 / 2.9, 128x64x64 26.4 / 7.3, 384x192x100
-// 164 / 113; Jacobi 72x20x100 17.7 / 4.6, 384x192x100 118 / 75; BiCGStab with
+// 139 / 87, 4000x80x80 409 / 305; Jacobi 72x20x100 17.7 / 4.6, 384x192x100
+// 93 / 50, 4000x80x80 285 / 169; BiCGStab with
 // the step around it, 40x20x20 44 / 25, 100x40x33 74 / 29, 131x75x53 93 / 58.
 //
 // Cell values are computed with the launched kernels' operations in their
 // order (poisson_math.cuh), or on the off-diagonal part where the cells are in
 // registers; sums differ in their order.
 //
-// A block whose barrier does not complete within its polls marks the solve's
-// state and leaves; the others leave at their next barrier.  A straggler may
+// A block whose barrier does not complete within BARRIER_POLLS polls marks the
+// solve's state and leaves; the others leave at their next barrier.  A straggler may
 // still find a barrier complete that another block gave up, so the mark is
 // never written over (finish), and the host reports DALM_ERR_DEVICE_WAIT
 // whatever else the state says.
@@ -41,7 +42,8 @@ namespace dalm {
 
 namespace {
 
-constexpr int RT = 512;  // threads of the sweep kernels
+constexpr int RT = 512;                       // threads of the sweep kernels
+constexpr unsigned BARRIER_POLLS = 1u << 21;  // about a second
 
 // The grid's barrier and sums.  One thread of a block adds 1 to a counter
 // (release) and polls it (acquire) until every block has: 2441 cycles over 148
@@ -53,10 +55,9 @@ constexpr int RT = 512;  // threads of the sweep kernels
 struct GridSync {
     unsigned *count;  // [0] arrivals, [1] failed; zeroed before the launch
     double2 *part;    // [2][gridDim.x]
-    unsigned polls;   // of one wait at most
     unsigned goal = 0;
     int set = 0;
-    __device__ GridSync(unsigned *c, double *p, unsigned limit) : count(c), part((double2 *)p), polls(limit) {}
+    __device__ GridSync(unsigned *c, double *p) : count(c), part((double2 *)p) {}
     static __device__ __forceinline__ unsigned load(const unsigned *p) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -67,7 +68,7 @@ struct GridSync {
         goal += gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         for (unsigned n = 0; (int)(load(count) - goal) < 0;) {
-            if (++n >= polls || ((n & 255u) == 0 && load(count + 1))) {
+            if (++n >= BARRIER_POLLS || ((n & 255u) == 0 && load(count + 1))) {
                 atomicExch(count + 1, 1u);
                 return false;
             }
@@ -267,7 +268,7 @@ __device__ __forceinline__ void finish(const KrylovState &S, KrylovState *st, bo
 // red cells of the other time level.
 __global__ void __launch_bounds__(RT, 1)
 k_resident_sor(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, const double *b, double w,
-               long long budget, double *part, unsigned *sync, unsigned polls, KrylovState *st) {
+               long long budget, double *part, unsigned *sync, KrylovState *st) {
     constexpr int U = 4;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
@@ -276,7 +277,7 @@ k_resident_sor(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, const
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part, polls);
+    GridSync grid(sync, part);
     double *cur = x, *nxt = tmp;  // red cells
     double black = 0.0;           // this thread's squared residuals at the black cells
     bool ok = true;
@@ -368,14 +369,14 @@ template <bool ONE>  // ONE: a single block, the packed arrays in its shared mem
 __global__ void __launch_bounds__(RT, 1)
 k_resident_sor_regs(Grid g, PoissonCoef C, Box box, Packed Q, double *x, double *red, double *blk,
                     const double *b, double w, long long budget, double *part, unsigned *sync,
-                    unsigned polls, KrylovState *st) {
+                    KrylovState *st) {
     constexpr int U = SOR_UI;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part, polls);
+    GridSync grid(sync, part);
     if (ONE) {
         red = resident_smem + 3 * (Q.ni + U);
         blk = red + Q.total();
@@ -506,7 +507,7 @@ k_resident_sor_regs(Grid g, PoissonCoef C, Box box, Packed Q, double *x, double 
 // Up to `budget` Jacobi iterations from x; tmp holds the other iterate.
 __global__ void __launch_bounds__(RT, 1)
 k_resident_jacobi(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, const double *b,
-                  long long budget, double *part, unsigned *sync, unsigned polls, KrylovState *st) {
+                  long long budget, double *part, unsigned *sync, KrylovState *st) {
     constexpr int U = 4;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
@@ -515,7 +516,7 @@ k_resident_jacobi(Grid g, PoissonCoef C, Cells cells, double *x, double *tmp, co
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part, polls);
+    GridSync grid(sync, part);
     double *cur = x, *nxt = tmp;
     bool ok = true;
     for (long long n = 0;; n++) {
@@ -609,13 +610,13 @@ struct Columns {
 template <int U, bool MEM>
 __global__ void __launch_bounds__(RT, 1)
 k_resident_bicg(Grid g, PoissonCoef C, Columns Q, PoissonBufs B, long long budget, double *part,
-                unsigned *sync, unsigned polls, KrylovState *st) {
+                unsigned *sync, KrylovState *st) {
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part, polls);
+    GridSync grid(sync, part);
     const Box &bx = Q.box;
     const int ni = bx.hi[0] - bx.lo[0];
     double *ci = resident_smem;  // coefficients along i, 0 past the interior
@@ -796,7 +797,7 @@ __device__ __forceinline__ void relax_color(const Domain &D, double *z, const do
 // update of v.
 __global__ void __launch_bounds__(RT, 1)
 k_resident_bicg_sor(Grid g, PoissonCoef C, Cells cells, PoissonBufs B, int sweeps, double w,
-                    long long budget, double *part, unsigned *sync, unsigned polls, KrylovState *st) {
+                    long long budget, double *part, unsigned *sync, KrylovState *st) {
     constexpr int U = 4;
     extern __shared__ double resident_smem[];
     __shared__ KrylovState S;
@@ -805,7 +806,7 @@ k_resident_bicg_sor(Grid g, PoissonCoef C, Cells cells, PoissonBufs B, int sweep
     if (threadIdx.x == 0) S = *st;
     __syncthreads();
     if (S.done) return;
-    GridSync grid(sync, part, polls);
+    GridSync grid(sync, part);
     bool ok = true;
     // v = update(c), z = M^-1 v, av = A z; v's sums with f: <f, av> or <av, v>, <av, av>
     auto half = [&](auto update, double *vv, double *z, double *av, const double *f, auto fin) {
@@ -877,7 +878,6 @@ constexpr size_t AXIS_SMEM = 200 * 1024, PACKED_SMEM = 150 * 1024, RESIDENT_SMEM
 template <typename K, typename... Args>
 bool cooperative(const LaunchCtx &L, K kernel, int blocks, int threads, size_t smem, Args... args) {
     void *ptrs[] = {(void *)&args...};
-    allow_shared(kernel, RESIDENT_SMEM);
     L.pre(KK_RESIDENT);
     const cudaError_t e =
         cudaLaunchCooperativeKernel((const void *)kernel, dim3(blocks), dim3(threads), ptrs, smem, L.s);
@@ -896,7 +896,7 @@ bool resident_bicg(const LaunchCtx &L, const Grid &g, const PoissonCoef &C, cons
                    KrylovState *st) {
     const Columns Q = Columns::make(cfg.seg.box, U);
     return cooperative(L, k_resident_bicg<U, MEM>, (int)((Q.threads + RT - 1) / RT), RT,
-                       3 * sizeof(double) * (size_t)(g.ni() + U), g, C, Q, B, budget, part, sync, cfg.wait_polls, st);
+                       3 * sizeof(double) * (size_t)(g.ni() + U), g, C, Q, B, budget, part, sync, st);
 }
 
 }  // namespace
@@ -914,12 +914,31 @@ bool resident_available(const PoissonConfig &cfg, const Grid &g) {
            AxisCoef::bytes(g) <= AXIS_SMEM;
 }
 
+void prepare_resident(const PoissonConfig &cfg) {
+    if (cfg.method == PM_SOR) {
+        allow_shared(k_resident_sor_regs<true>, RESIDENT_SMEM);
+        allow_shared(k_resident_sor_regs<false>, RESIDENT_SMEM);
+        allow_shared(k_resident_sor, RESIDENT_SMEM);
+    } else if (cfg.method == PM_JACOBI) {
+        allow_shared(k_resident_jacobi, RESIDENT_SMEM);
+    } else if (cfg.pc == PC_SOR) {
+        allow_shared(k_resident_bicg_sor, RESIDENT_SMEM);
+    } else {
+        allow_shared(k_resident_bicg<1, false>, RESIDENT_SMEM);
+        allow_shared(k_resident_bicg<2, false>, RESIDENT_SMEM);
+        allow_shared(k_resident_bicg<4, false>, RESIDENT_SMEM);
+        allow_shared(k_resident_bicg<8, true>, RESIDENT_SMEM);
+    }
+}
+
 bool launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef &C,
                            const PoissonBufs &B, const PoissonConfig &cfg, long long budget,
                            double *part, unsigned *sync, KrylovState *st) {
     const Cells cells = Cells::make(cfg.seg.box);
     const unsigned threads = (unsigned)cfg.sm_count * RT;
     DALM_CUDA(cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), L.s));
+    // a count that no number of arrivals completes
+    if (cfg.stall_waits) DALM_CUDA(cudaMemsetAsync(sync, 0xc0, sizeof(unsigned), L.s));
     if (cfg.method == PM_BICG && cfg.pc == PC_JACOBI) {
         // the fewest planes per thread that fit the grid on the device
         auto fits = [&](int planes) { return Columns::make(cfg.seg.box, planes).threads <= threads; };
@@ -938,19 +957,18 @@ bool launch_resident_solve(const LaunchCtx &L, const Grid &g, const PoissonCoef 
         const size_t axis = 3 * sizeof(double) * (size_t)(Q.ni + SOR_UI), packed = 2 * sizeof(double) * (size_t)Q.total();
         if (Q.threads <= RT && packed <= PACKED_SMEM)
             return cooperative(L, k_resident_sor_regs<true>, 1, RT, axis + packed, g, C, cfg.seg.box, Q, B.x, B.tp,
-                               B.ts, B.b, cfg.relax, budget, part, sync, cfg.wait_polls, st);
+                               B.ts, B.b, cfg.relax, budget, part, sync, st);
         if (Q.threads <= threads)
             return cooperative(L, k_resident_sor_regs<false>, (int)((Q.threads + RT - 1) / RT), RT, axis, g, C,
-                               cfg.seg.box, Q, B.x, B.tp, B.ts, B.b, cfg.relax, budget, part, sync, cfg.wait_polls,
-                               st);
+                               cfg.seg.box, Q, B.x, B.tp, B.ts, B.b, cfg.relax, budget, part, sync, st);
         return cooperative(L, k_resident_sor, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, cfg.relax, budget,
-                           part, sync, cfg.wait_polls, st);
+                           part, sync, st);
     }
     if (cfg.method == PM_JACOBI)
         return cooperative(L, k_resident_jacobi, blocks, RT, smem, g, C, cells, B.x, B.tp, B.b, budget, part,
-                           sync, cfg.wait_polls, st);
+                           sync, st);
     return cooperative(L, k_resident_bicg_sor, blocks, RT, smem, g, C, cells, B, cfg.pc_sweeps, cfg.pc_relax,
-                       budget, part, sync, cfg.wait_polls, st);
+                       budget, part, sync, st);
 }
 
 }  // namespace dalm
