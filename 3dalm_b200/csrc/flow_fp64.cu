@@ -106,11 +106,6 @@ __device__ __forceinline__ double smagorinsky(const StepParams &P, Vec3<const do
     return P.filter2[c] * shear;
 }
 
-__device__ __forceinline__ bool interior(const Grid &g, int i, int j, int k) {
-    return i >= g.gc && i < g.nx - g.gc && j >= g.gc && j < g.ny - g.gc && k >= g.gc &&
-           k < g.nz - g.gc;
-}
-
 // ---------------------------------------------------------------- predictor
 //
 // cpy_array(Uold, U) + calc_intermediate_U (src/solver.h:1042-1053,

@@ -22,7 +22,7 @@ namespace dalm {
 constexpr int WIDE_HK = 4, WIDE_HJ = 3;
 
 // `half` boxes of the BiCGStab half-iterations (poisson_half.cuh): W x ROWS
-// cells, for grids above or up to 32 cells high
+// cells, for grids above or up to 32 cells high; FP64 fields only
 constexpr int WIDE_BOX_K = 72, WIDE_BOX_J = 21, NARROW_BOX_K = 40, NARROW_BOX_J = 24;
 
 struct FieldMaps {
@@ -53,12 +53,6 @@ __device__ __forceinline__ void fence_barrier_init() {
 
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// orders this thread's global writes (and those it has acquired) with
-// TMA loads of the same memory
-__device__ __forceinline__ void fence_proxy_global() {
-    asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {

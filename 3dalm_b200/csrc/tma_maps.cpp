@@ -45,13 +45,15 @@ FieldMaps make_field_maps(const Grid &g, const void *base, int elem_bytes) {
     if (elem_bytes != 4 && elem_bytes != 8) throw std::invalid_argument("element size");
     if (((uintptr_t)base) % 16 != 0) throw std::invalid_argument("TMA base not 16-byte aligned");
     if ((g.sy * elem_bytes) % 16 != 0) throw std::invalid_argument("row pitch not 16-byte multiple");
-    FieldMaps m;
+    FieldMaps m{};
     int h = 16 / elem_bytes;
     encode(&m.halo, g, base, elem_bytes, (cuuint32_t)(TK + 2 * h), (cuuint32_t)(TJ + 2));
     encode(&m.plain, g, base, elem_bytes, (cuuint32_t)TK, (cuuint32_t)TJ);
     encode(&m.wide, g, base, elem_bytes, (cuuint32_t)(TK + 2 * WIDE_HK), (cuuint32_t)(TJ + 2 * WIDE_HJ));
-    const bool high = g.nk() > NARROW_BOX_K - 8;
-    encode(&m.half, g, base, elem_bytes, high ? WIDE_BOX_K : NARROW_BOX_K, high ? WIDE_BOX_J : NARROW_BOX_J);
+    if (elem_bytes == 8) {
+        const bool high = g.nk() > NARROW_BOX_K - 8;
+        encode(&m.half, g, base, elem_bytes, high ? WIDE_BOX_K : NARROW_BOX_K, high ? WIDE_BOX_J : NARROW_BOX_J);
+    }
     return m;
 }
 

@@ -127,7 +127,13 @@ typedef struct {
                              convergence checks (0: automatic)           */
     int use_graphs;       /* 1: replay iteration batches as CUDA graphs  */
     int profile;          /* 1: time every kernel launch with CUDA events
-                             (dalm_get_kernel_timings)                   */
+                             (dalm_get_kernel_timing).  Solves that run
+                             whole as one kernel, and the multigrid levels
+                             that run as one, are launched loop by loop
+                             with it: the kinds then show the launched
+                             form, which is slower on grids that take the
+                             other, and the fields differ by rounding
+                             (FP64 solves) or not at all (multigrid)     */
     int reference_sums;   /* 1: every global sum (Krylov dots, norms,
                              divergence norm) in the reference's serial
                              cell order instead of a parallel tree, and
