@@ -805,6 +805,9 @@ struct dalm_handle {
             h_kst[q].wait_error = 0;
             DALM_CUDA(cudaMemsetAsync(&d_kst[q].wait_error, 0, sizeof(int), stream));
         }
+        // a block that gave up took no ticket, and the next reduction would
+        // take an early block for its last
+        DALM_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), stream));
         throw DeviceWaitError("a bounded wait in the Poisson solver ran out");
     }
     // Enqueues iterations of solve `which` in batches and polls the device's
